@@ -18,12 +18,27 @@
 // Scratch areas inside the context (grown on demand, never shrunk).
 enum { MOE_SCR_SCATTER = 0, MOE_SCR_LAYER = 1, MOE_SCR_STAGE = 2, MOE_SCR_EP = 3, MOE_SCR_COUNT = 4 };
 
+// Tensor maps already made, by what they describe: a hash picks a set of MOE_TMAP_WAYS entries, a full set gives up its
+// entries in turn.  512 entries hold the weights of a 48-layer stack (3 per layer) beside everything else of a context;
+// callers get a copy, so an entry that is given up later does no harm.
+#define MOE_TMAP_SETS 128u
+#define MOE_TMAP_WAYS 4u
 struct moe_tmap_entry {
+    const void *ptr;  // NULL: free
+    uint64_t rows, cols;
+    uint32_t box_rows, kind;  // kind 0: plain 2-D; 1: gate/up interleaved 4-D
+    CUtensorMap map;
+};
+// The same for the token operand of the weight-stationary products: boxes of 16, 32, ... 128 rows of one matrix.
+#define MOE_XMAP_BOXES 8u
+#define MOE_XMAP_SETS 8u
+struct moe_xmaps {
+    CUtensorMap m[MOE_XMAP_BOXES];
+};
+struct moe_xmap_entry {
     const void *ptr;
     uint64_t rows, cols;
-    uint32_t box_rows, box_cols;
-    uint32_t kind;  // 0: plain 2-D; 1: gate/up interleaved 4-D
-    CUtensorMap map;
+    moe_xmaps maps;
 };
 
 struct moe_ep_state;  // moe_ep.cu
@@ -41,8 +56,9 @@ struct moe_cuda_ctx {
     uint32_t *dev_status_dev;
     void *scratch[MOE_SCR_COUNT];
     size_t scratch_bytes[MOE_SCR_COUNT];
-    moe_tmap_entry tmaps[128];
-    int n_tmaps, next_tmap;
+    moe_tmap_entry tmaps[MOE_TMAP_SETS][MOE_TMAP_WAYS];
+    moe_xmap_entry xmaps[MOE_XMAP_SETS][MOE_TMAP_WAYS];
+    uint8_t next_tmap[MOE_TMAP_SETS], next_xmap[MOE_XMAP_SETS];
     void *encode_tiled;  // cuTensorMapEncodeTiled, resolved at create
     bool prof;
     cudaEvent_t ev[MOE_PROF_STAGES + 1];
@@ -52,6 +68,7 @@ struct moe_cuda_ctx {
     uint64_t launches;
     int fail_alloc_countdown;
     bool mm_attr_set[4];
+    bool kd_attr_set;
     uint32_t *ticket;  // device word, zero between kernels: "last block done" counter
     bool sw_attr_set[8];
     moe_ep_state *ep;
@@ -62,12 +79,12 @@ void moe_fail(moe_cuda_ctx *c, int code, const char *fmt, ...);
 void *moe_scratch(moe_cuda_ctx *c, int area, size_t bytes);
 bool moe_poll_device_status(moe_cuda_ctx *c);
 void moe_ep_teardown(moe_cuda_ctx *c);
-const CUtensorMap *moe_tmap_2d_f16(moe_cuda_ctx *c, const void *ptr, uint64_t rows, uint64_t cols,
-                                   uint32_t box_rows, uint32_t box_cols);
-
+// 2-D fp16 tensor map [rows x cols], box box_rows x 64.  False: the context has failed.
+bool moe_tmap_2d_f16(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows);
+bool moe_tmap_tokens_f16(moe_cuda_ctx *c, moe_xmaps *out, const void *ptr, uint64_t rows, uint64_t cols);
 // 4-D fp16 tensor map over an expert bank [experts][2][inter][k] (gate rows then up rows per expert) whose
 // box (64 k, 2, 64 inter, 1 expert) lands in shared memory as 128 rows: row 2i = gate row i, row 2i+1 = up row i.
-const CUtensorMap *moe_tmap_gate_up_f16(moe_cuda_ctx *c, const void *ptr, uint32_t experts, uint32_t inter, uint32_t k);
+bool moe_tmap_gate_up_f16(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint32_t experts, uint32_t inter, uint32_t k);
 
 #define MOE_LIVE(c) ((c) != NULL && (c)->status == MOE_OK)
 

@@ -287,82 +287,98 @@ extern "C" void moe_cuda_prof_read(moe_cuda_ctx_t *c, float ms[MOE_PROF_STAGES])
     }
 }
 
-// 2-D fp16 tensor map [rows x cols], row-major, swizzle = the box's row width (128 or 64 bytes), zero fill
-// outside the tensor; never multicast.  Cached per (pointer, shape, box).
+// Tensor maps: row-major fp16, boxes of 64 columns with a 128-byte swizzle, zero fill outside the tensor; never multicast.
 typedef CUresult (*moe_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                   CUtensorMapFloatOOBfill);
 
-const CUtensorMap *moe_tmap_2d_f16(moe_cuda_ctx *c, const void *ptr, uint64_t rows, uint64_t cols,
-                                   uint32_t box_rows, uint32_t box_cols) {
-    if (!MOE_LIVE(c)) return NULL;
-    for (int i = 0; i < c->n_tmaps; i += 1) {
-        moe_tmap_entry *t = &c->tmaps[i];
-        if (t->kind == 0 && t->ptr == ptr && t->rows == rows && t->cols == cols && t->box_rows == box_rows && t->box_cols == box_cols) {
-            return &t->map;
-        }
-    }
-    if (((uintptr_t)ptr & 15) != 0 || (cols * 2) % 16 != 0 || (box_cols * 2 != 128 && box_cols * 2 != 64) || box_rows > 256 || rows == 0) {
+static bool moe_encode(moe_cuda_ctx *c, CUtensorMap *out, uint32_t rank, const void *ptr, const cuuint64_t *dims,
+                       const cuuint64_t *strides, const cuuint32_t *box) {
+    static const cuuint32_t ones[4] = {1, 1, 1, 1};
+    CUresult r = ((moe_encode_fn)c->encode_tiled)(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, (void *)ptr, dims, strides, box, ones,
+                                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) moe_fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
+    return r == CUDA_SUCCESS;
+}
+
+static uint32_t moe_tmap_hash(const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+    uint64_t h = ((uint64_t)(uintptr_t)ptr >> 4) ^ (rows << 24) ^ (cols << 40) ^ ((uint64_t)box_rows << 56);
+    return (uint32_t)((h * 0x9e3779b97f4a7c15ull) >> 40);
+}
+
+static bool moe_tmap_encode_2d(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+    if (((uintptr_t)ptr & 15) != 0 || ptr == NULL || (cols * 2) % 16 != 0 || box_rows > 256 || rows == 0) {
         moe_fail(c, MOE_ERR_ARG, "tensor map: base %p rows %llu cols %llu not TMA-addressable", ptr,
                  (unsigned long long)rows, (unsigned long long)cols);
-        return NULL;
+        return false;
     }
-    int at = c->n_tmaps < 128 ? c->n_tmaps++ : (c->next_tmap++ & 127);
-    moe_tmap_entry *t = &c->tmaps[at];
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
-    cuuint32_t box[2] = {box_cols, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = ((moe_encode_fn)c->encode_tiled)(&t->map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)ptr, dims,
-                                                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                                  box_cols * 2 == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        moe_fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
-        c->n_tmaps = at < c->n_tmaps ? c->n_tmaps : at;
-        t->ptr = NULL;
-        return NULL;
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {64, box_rows};
+    return moe_encode(c, out, 2, ptr, dims, strides, box);
+}
+
+// One entry of `kind`: the cached one, or a new one in its place.
+static bool moe_tmap_get(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t kind) {
+    if (!MOE_LIVE(c)) return false;
+    const uint32_t set = moe_tmap_hash(ptr, rows, cols, box_rows + kind) % MOE_TMAP_SETS;
+    for (uint32_t i = 0; i < MOE_TMAP_WAYS; i += 1) {
+        moe_tmap_entry *t = &c->tmaps[set][i];
+        if (t->ptr == ptr && t->rows == rows && t->cols == cols && t->box_rows == box_rows && t->kind == kind && ptr != NULL) {
+            memcpy(out, &t->map, sizeof(*out));
+            return true;
+        }
     }
+    if (kind == 0) {
+        if (!moe_tmap_encode_2d(c, out, ptr, rows, cols, box_rows)) return false;
+    } else {  // gate/up bank: rows = experts, box_rows = inter
+        const cuuint64_t inter = box_rows;
+        const cuuint64_t dims[4] = {cols, 2, inter, rows};
+        const cuuint64_t strides[3] = {inter * cols * 2, cols * 2, 2 * inter * cols * 2};
+        const cuuint32_t box[4] = {64, 2, 64, 1};
+        if (!moe_encode(c, out, 4, ptr, dims, strides, box)) return false;
+    }
+    moe_tmap_entry *t = &c->tmaps[set][c->next_tmap[set]++ % MOE_TMAP_WAYS];
     t->ptr = ptr;
     t->rows = rows;
     t->cols = cols;
     t->box_rows = box_rows;
-    t->box_cols = box_cols;
-    t->kind = 0;
-    return &t->map;
+    t->kind = kind;
+    memcpy(&t->map, out, sizeof(*out));
+    return true;
 }
 
-const CUtensorMap *moe_tmap_gate_up_f16(moe_cuda_ctx *c, const void *ptr, uint32_t experts, uint32_t inter, uint32_t k) {
-    if (!MOE_LIVE(c)) return NULL;
-    for (int i = 0; i < c->n_tmaps; i += 1) {
-        moe_tmap_entry *t = &c->tmaps[i];
-        if (t->kind == 1 && t->ptr == ptr && t->rows == experts && t->cols == k && t->box_rows == inter) return &t->map;
-    }
-    if (((uintptr_t)ptr & 15) != 0 || k % 8u != 0 || inter % 64u != 0 || experts == 0) {
+bool moe_tmap_2d_f16(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+    return moe_tmap_get(c, out, ptr, rows, cols, box_rows, 0);
+}
+
+bool moe_tmap_gate_up_f16(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, uint32_t experts, uint32_t inter, uint32_t k) {
+    if (!MOE_LIVE(c)) return false;
+    if (((uintptr_t)ptr & 15) != 0 || ptr == NULL || k % 8u != 0 || inter % 64u != 0 || experts == 0) {
         moe_fail(c, MOE_ERR_ARG, "tensor map: gate/up bank %p experts %u inter %u k %u not TMA-addressable", ptr, experts, inter, k);
-        return NULL;
+        return false;
     }
-    int at = c->n_tmaps < 128 ? c->n_tmaps++ : (c->next_tmap++ & 127);
-    moe_tmap_entry *t = &c->tmaps[at];
-    cuuint64_t dims[4] = {k, 2, inter, experts};
-    cuuint64_t strides[3] = {(cuuint64_t)inter * k * 2, (cuuint64_t)k * 2, (cuuint64_t)2 * inter * k * 2};
-    cuuint32_t box[4] = {64, 2, 64, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = ((moe_encode_fn)c->encode_tiled)(&t->map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void *)ptr, dims, strides, box,
-                                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        moe_fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled (gate/up bank) failed: %d", (int)r);
-        t->ptr = NULL;
-        return NULL;
+    return moe_tmap_get(c, out, ptr, experts, k, inter, 1);
+}
+
+bool moe_tmap_tokens_f16(moe_cuda_ctx *c, moe_xmaps *out, const void *ptr, uint64_t rows, uint64_t cols) {
+    if (!MOE_LIVE(c)) return false;
+    const uint32_t set = moe_tmap_hash(ptr, rows, cols, 0) % MOE_XMAP_SETS;
+    for (uint32_t i = 0; i < MOE_TMAP_WAYS; i += 1) {
+        moe_xmap_entry *t = &c->xmaps[set][i];
+        if (t->ptr == ptr && t->rows == rows && t->cols == cols && ptr != NULL) {
+            memcpy(out, &t->maps, sizeof(*out));
+            return true;
+        }
     }
+    for (uint32_t i = 0; i < MOE_XMAP_BOXES; i += 1) {
+        if (!moe_tmap_encode_2d(c, &out->m[i], ptr, rows, cols, 16u * (i + 1u))) return false;
+    }
+    moe_xmap_entry *t = &c->xmaps[set][c->next_xmap[set]++ % MOE_TMAP_WAYS];
     t->ptr = ptr;
-    t->rows = experts;
-    t->cols = k;
-    t->box_rows = inter;
-    t->box_cols = 64;
-    t->kind = 1;
-    return &t->map;
+    t->rows = rows;
+    t->cols = cols;
+    memcpy(&t->maps, out, sizeof(*out));
+    return true;
 }

@@ -23,13 +23,10 @@ namespace {
 
 using namespace moe_tc;
 
-#ifndef MM_BK
-#define MM_BK 64
-#endif
 // K step per stage: 64 (128-byte rows, 128-byte swizzle, 4 stages of 48 KB).  32 (64-byte rows, 64-byte
-// swizzle, 8 stages of 24 KB) also builds and passes the parity tests but is 40 % slower on B200: its
-// half-line row requests stream worse, which outweighs the finer stage recycling.
-constexpr uint32_t BM = 128, BN = 256, BK = MM_BK, STAGES = 256 / MM_BK;
+// swizzle, 8 stages of 24 KB) is 40 % slower on B200: its half-line row requests stream worse, which outweighs
+// the finer stage recycling.
+constexpr uint32_t BM = 128, BN = 256, BK = 64, STAGES = 4;
 constexpr uint32_t ROW_BYTES = BK * 2;          // bytes of one operand row per stage = the swizzle span
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t BH_BYTES = 128 * BK * 2;     // half of the B tile
@@ -196,8 +193,7 @@ moe_mm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                     if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     tc_fence_after();
                     uint32_t base = stage0 + s * STAGE_BYTES;
-                    uint64_t ad = BK == 64 ? umma_desc(base) : umma_desc_sw64(base);
-                    uint64_t bd = BK == 64 ? umma_desc(base + A_BYTES) : umma_desc_sw64(base + A_BYTES);
+                    uint64_t ad = umma_desc(base), bd = umma_desc(base + A_BYTES);
 #pragma unroll
                     for (uint32_t kk = 0; kk < BK / 16; kk += 1) {
                         // +32 bytes per K=16 step inside the 128-byte swizzle row
@@ -223,8 +219,8 @@ moe_mm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         constexpr uint32_t CPR = ROW_BYTES / 16u, RPI = 128u / CPR, NJ = BM / RPI;
         const uint32_t g = (warp - 6u) * 32u + lane;
         const uint32_t sub = g / CPR, ch = g % CPR;
-        // swizzle as TMA writes it: 128-byte rows: chunk ^ (row % 8); 64-byte rows: chunk ^ ((row / 2) % 4)
-        const uint32_t dst_off = sub * ROW_BYTES + ((ch ^ (BK == 64 ? (sub & 7u) : ((sub >> 1) & 3u))) << 4);
+        // swizzle as TMA writes it: chunk ^ (row % 8)
+        const uint32_t dst_off = sub * ROW_BYTES + ((ch ^ (sub & 7u)) << 4);
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (uint32_t w = blockIdx.x; w < total && ok; w += gridDim.x) {
@@ -351,13 +347,13 @@ moe_mm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 }
 
 template <int MODE, bool GATHER>
-void mm_launch(moe_cuda_ctx *c, const CUtensorMap *tmA, const CUtensorMap *tmB, const MmArgs &a, uint32_t grid) {
+void mm_launch(moe_cuda_ctx *c, const CUtensorMap &tmA, const CUtensorMap &tmB, const MmArgs &a, uint32_t grid) {
     const int slot = GATHER ? 3 : MODE;
     if (!c->mm_attr_set[slot]) {
         MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_mm_kernel<MODE, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
         c->mm_attr_set[slot] = true;
     }
-    moe_mm_kernel<MODE, GATHER><<<grid, MM_THREADS + (GATHER ? 128 : 0), MM_SMEM, c->stream>>>(*tmA, *tmB, a);
+    moe_mm_kernel<MODE, GATHER><<<grid, MM_THREADS + (GATHER ? 128 : 0), MM_SMEM, c->stream>>>(tmA, tmB, a);
     MOE_LAUNCHED(c);
 }
 
@@ -377,9 +373,8 @@ void moe_launch_mm(moe_cuda_ctx *c, int mode, const void *A, const void *B, void
     MOE_REQUIRE(c, src_row == NULL || (mode == MOE_MM_SWIGLU_F16 && ((uintptr_t)A & 15) == 0), "mm: row gather is for the gate_up product");
     MOE_REQUIRE(c, (sa == MDA_PC_NO_SLOT && sb == MDA_PC_NO_SLOT) || amax != NULL, "mm: scale slot without amax");
     MOE_REQUIRE(c, ((uintptr_t)C & 15) == 0, "mm: C not 16-byte aligned");
-    const CUtensorMap *tmA = moe_tmap_2d_f16(c, A, a_rows, k, 128, BK);
-    const CUtensorMap *tmB = moe_tmap_2d_f16(c, B, (uint64_t)experts_in_B * n, k, 128, BK);
-    if (tmA == NULL || tmB == NULL) return;
+    CUtensorMap tmA, tmB;
+    if (!moe_tmap_2d_f16(c, &tmA, A, a_rows, k, 128) || !moe_tmap_2d_f16(c, &tmB, B, (uint64_t)experts_in_B * n, k, 128)) return;
     MmArgs a;
     a.C = C;
     a.amax = amax;

@@ -19,8 +19,6 @@
 // fp16 store are the epilogue.
 // Every spin on an mbarrier is bounded; on timeout the kernel records
 // MOE_ERR_TIMEOUT in the context's status word and unwinds.
-#include <stdlib.h>
-
 #include "moe_tc.cuh"
 
 namespace {
@@ -68,9 +66,6 @@ struct WsArgs {
     uint32_t ldc;              // row stride of C in elements
     uint32_t *status;
     uint64_t wait_ns;
-    unsigned long long *prof;  // per CTA 8 cycle counters, or NULL
-    unsigned long long *trace; // profiling builds: event trace, or NULL
-    uint32_t dbg;              // profiling builds only: 1 no MMA, 2 no token loads, 4 no weight loads, 8 no stores, 32 no epilogue
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -162,21 +157,6 @@ __device__ __forceinline__ uint32_t x_rows_loaded(uint32_t half) {
     for (uint32_t done = 0; done < half; done += x_box_rows(half - done)) rows += x_box_rows(half - done);
     return rows;
 }
-struct XMaps {
-    CUtensorMap m[8];  // boxes of 16, 32, ... 128 token rows
-#ifdef MOE_WS_PROF
-    CUtensorMap wc;    // experiment: the weight bank as rows of 512 bytes, 16 KB contiguous per box
-#endif
-};
-
-// Profiling builds: event trace of the first two CTAs (one pair), 8 timestamps per K step, 512 K steps.
-#define WS_TRACE_STEPS 512u
-__device__ __forceinline__ void ws_trace(unsigned long long *trace, uint32_t step, uint32_t slot) {
-    if (trace != NULL && blockIdx.x < 2u && step < WS_TRACE_STEPS) {
-        trace[((size_t)blockIdx.x * WS_TRACE_STEPS + step) * 8u + slot] = (unsigned long long)clock64();
-    }
-}
-
 struct WsItem {
     uint32_t e, row0, ntok, nvalid, ft;
 };
@@ -191,9 +171,9 @@ __device__ __forceinline__ void ws_item(const WsArgs &a, uint32_t w, uint32_t ft
     it.nvalid = ch.w;
 }
 
-template <int MODE, int PAIR, bool PROF>
+template <int MODE, int PAIR>
 __global__ void __launch_bounds__(WS_THREADS, 1)
-moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ XMaps tmX, WsArgs a) {
+moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ moe_xmaps tmX, WsArgs a) {
     using G = Geo<PAIR>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -209,8 +189,6 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const uint32_t total = *a.n_chunks * ft_count;
     const uint32_t kblocks = (a.k + BK - 1) / BK;
     const uint32_t cluster_id = blockIdx.x / PAIR, n_clusters = gridDim.x / PAIR;
-    long long t_begin = 0;
-    if (PROF) t_begin = clock64();
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < G::STAGES; s += 1) {
@@ -254,61 +232,37 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (lane == 0) {
             const bool wprod = warp == 0 || (warp >= 7 && (warp & 1u) != 0);
             const uint32_t turn_of = warp < 7 ? 0u : (warp - 5u) / 2u;  // 0, 1, 2: which K steps this thread takes
-            const uint32_t dbg = PROF ? a.dbg : 0u;
-            uint32_t s = 0, ph = 0, issued = 0, last_par = 0, step = 0, gstep = 0;
-            long long waited = 0, issue_busy = 0;
+            uint32_t s = 0, ph = 0, issued = 0, last_par = 0, gstep = 0;
             bool ok = true;
-            for (uint32_t w = cluster_id; w < total && ok && !(dbg & 512u); w += n_clusters) {
+            for (uint32_t w = cluster_id; w < total && ok; w += n_clusters) {
                 WsItem it;
                 ws_item(a, w, ft_count, it);
                 const uint32_t half = it.ntok / PAIR;            // token rows this CTA loads
-                const uint32_t xbytes = (dbg & 2u) ? 0u : x_rows_loaded(half) * (BK * 2u);
-                const uint32_t wbytes = (dbg & 4u) ? 0u : W_BYTES;
+                const uint32_t xbytes = x_rows_loaded(half) * (BK * 2u);
                 const int32_t f0 = (int32_t)((it.ft * PAIR + rank) * (MODE == MOE_MM_SWIGLU_F16 ? 64u : 128u));
                 const int32_t xrow = (int32_t)(it.row0 + rank * half);
                 for (uint32_t kb = 0; kb < kblocks; kb += 1, gstep += 1) {
                     if (gstep % NPROD != turn_of) continue;
                     s = gstep % G::STAGES;
                     ph = (gstep / G::STAGES) & 1u;
-                    long long t0 = 0;
-                    if (PROF) t0 = clock64();
                     if (!mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort, a.status, wprod ? 11 : 15, a.wait_ns)) {
                         ok = false;
                         break;
-                    }
-                    long long t1 = 0;
-                    if (PROF) {
-                        t1 = clock64();
-                        waited += t1 - t0;
-                        ws_trace(a.trace, step, wprod ? 0u : 2u);
                     }
                     const uint32_t base = stage0 + s * G::STAGE_BYTES;
                     const int32_t kc = (int32_t)(kb * BK);
                     const uint32_t full = PAIR == 2 ? map_to_cta(smem_u32(&bars->full[s]), 0) : smem_u32(&bars->full[s]);
                     if (wprod) {
-                        if (rank == 0) mbar_expect_tx(smem_u32(&bars->full[s]), (uint32_t)PAIR * (wbytes + xbytes));
-                        if (PROF && (dbg & 64u)) {
-#ifdef MOE_WS_PROF
-                            // experiment: same bytes, but each tile one contiguous 16 KB piece of the bank
-                            const uint32_t tile = (it.e * ft_count * PAIR + it.ft * PAIR + rank) * kblocks + kb;
-                            tma_2d<PAIR>(base, &tmX.wc, full, 0, (int32_t)(tile * 32u));
-#endif
-                        } else if (wbytes != 0u) {
-                            if (MODE == MOE_MM_SWIGLU_F16) tma_4d<PAIR>(base, &tmW, full, kc, 0, f0, (int32_t)it.e);
-                            else tma_2d<PAIR>(base, &tmW, full, kc, (int32_t)(it.e * a.n) + f0);
-                        }
-                    } else if (xbytes != 0u) {
+                        if (rank == 0) mbar_expect_tx(smem_u32(&bars->full[s]), (uint32_t)PAIR * (W_BYTES + xbytes));
+                        if (MODE == MOE_MM_SWIGLU_F16) tma_4d<PAIR>(base, &tmW, full, kc, 0, f0, (int32_t)it.e);
+                        else tma_2d<PAIR>(base, &tmW, full, kc, (int32_t)(it.e * a.n) + f0);
+                    } else {
                         uint32_t done = 0;
                         while (done < half) {  // boxes of 16, 32, ... 128 token rows: at most 15 rows more than needed
                             const uint32_t rows = x_box_rows(half - done);
                             tma_2d<PAIR>(base + W_BYTES + done * (BK * 2u), &tmX.m[rows / 16u - 1u], full, kc, xrow + (int32_t)done);
                             done += rows;
                         }
-                    }
-                    if (PROF) {
-                        issue_busy += clock64() - t1;
-                        ws_trace(a.trace, step, wprod ? 1u : 3u);
-                        step += 1;
                     }
                     issued |= 1u << s;
                     last_par = (last_par & ~(1u << s)) | (ph << s);
@@ -322,10 +276,6 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     }
                 }
             }
-            if (PROF && a.prof != NULL && turn_of == 0) {
-                a.prof[blockIdx.x * 16u + (wprod ? 1u : 8u)] = (unsigned long long)waited;
-                a.prof[blockIdx.x * 16u + (wprod ? 9u : 10u)] = (unsigned long long)issue_busy;
-            }
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -334,49 +284,36 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         // elected lane issues; one look at the full barriers covers the whole ring (mbar_ring_wait).
         if (rank == 0) {
             uint32_t gstep = 0, n_item = 0, ready = 0;
-            long long wait_full = 0, wait_acc = 0;
             bool ok = true;
             for (uint32_t w = cluster_id; w < total && ok; w += n_clusters) {
                 WsItem it;
                 ws_item(a, w, ft_count, it);
                 const uint32_t as = n_item & 1u, aph = (n_item >> 1) & 1u;
-                long long t0 = 0;
-                if (PROF) t0 = clock64();
                 if (!mbar_wait(smem_u32(&bars->tmem_empty[as]), aph ^ 1u, abort, a.status, 12, a.wait_ns)) break;
-                if (PROF) wait_acc += clock64() - t0;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + as * MAX_TOK;
                 const uint32_t idesc = umma_idesc(128u * PAIR, it.ntok);
                 for (uint32_t kb = 0; kb < kblocks; kb += 1, gstep += 1) {
                     const uint32_t s = gstep % G::STAGES;
-                    if (PROF) t0 = clock64();
-                    if (!(PROF && (a.dbg & 512u)) && ((ready >> s) & 1u) == 0 &&
+                    if (((ready >> s) & 1u) == 0 &&
                         !mbar_ring_wait<G::STAGES>(bars->full, gstep, ready, abort, a.status, 13, a.wait_ns)) {
                         ok = false;
                         break;
                     }
                     ready &= ~(1u << s);
-                    if (PROF) {
-                        wait_full += clock64() - t0;
-                        if (lane == 0) ws_trace(a.trace, gstep, 4u);
-                    }
                     tc_fence_after();
                     const uint32_t base = stage0 + s * G::STAGE_BYTES;
                     const uint64_t ad = umma_desc(base), bd = umma_desc(base + W_BYTES);
                     if (elect_one()) {
-                        if (!(PROF && (a.dbg & 1u))) {
 #pragma unroll
-                            for (uint32_t kk = 0; kk < BK / 16; kk += 1) {
-                                if (PAIR == 2) umma_f16_pair(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-                                else umma_f16(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-                            }
+                        for (uint32_t kk = 0; kk < BK / 16; kk += 1) {
+                            if (PAIR == 2) umma_f16_pair(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                            else umma_f16(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
                         }
-                        if (PROF && (a.dbg & 512u)) {  // experiment: tensor pipe alone, nothing is loaded, no stage hand-off
-                        } else if (PAIR == 2) umma_commit_both(smem_u32(&bars->empty[s]));  // frees the stage in both CTAs
+                        if (PAIR == 2) umma_commit_both(smem_u32(&bars->empty[s]));  // frees the stage in both CTAs
                         else umma_commit(smem_u32(&bars->empty[s]));
                     }
                     __syncwarp();
-                    if (PROF && lane == 0) ws_trace(a.trace, gstep, 5u);
                 }
                 if (ok && elect_one()) {
                     if (PAIR == 2) umma_commit_both(smem_u32(&bars->tmem_full[as]));
@@ -384,12 +321,6 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 }
                 __syncwarp();
                 n_item += 1;
-            }
-            if (PROF && a.prof != NULL && lane == 0) {
-                a.prof[blockIdx.x * 16u + 2u] = (unsigned long long)wait_full;
-                a.prof[blockIdx.x * 16u + 3u] = (unsigned long long)wait_acc;
-                a.prof[blockIdx.x * 16u + 6u] = n_item;
-                a.prof[blockIdx.x * 16u + 7u] = gstep;
             }
         }
         __syncwarp();
@@ -399,26 +330,16 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const uint32_t ew = warp - 2u;   // 0..3: which rows of the turn-round tile this warp stores
         const uint32_t empty_leader = PAIR == 2 ? map_to_cta(smem_u32(&bars->tmem_empty[0]), 0) : smem_u32(&bars->tmem_empty[0]);
         uint32_t n_item = 0, tb = 0;
-        long long wait_acc = 0, busy = 0;
         for (uint32_t w = cluster_id; w < total; w += n_clusters) {
             WsItem it;
             ws_item(a, w, ft_count, it);
             const uint32_t as = n_item & 1u, aph = (n_item >> 1) & 1u;
-            long long t0 = 0;
-            if (PROF) t0 = clock64();
             bool ok = true;
             if (lane == 0) ok = mbar_wait(smem_u32(&bars->tmem_full[as]), aph, abort, a.status, 14, a.wait_ns);
             if (!epi_all(ok)) break;
-            long long t1 = 0;
-            if (PROF) {
-                t1 = clock64();
-                wait_acc += t1 - t0;
-            }
             tc_fence_after();
             const uint32_t taddr = tmem_base + as * MAX_TOK + ((q * 32u) << 16);
-            uint32_t nch = (it.ntok + ET - 1u) / ET;
-            if (PROF && (a.dbg & 8u)) it.nvalid = 0;
-            if (PROF && (a.dbg & 32u)) nch = 0;
+            const uint32_t nch = (it.ntok + ET - 1u) / ET;
             if (MODE == MOE_MM_SWIGLU_F16) {
                 // lane 2i holds gate feature i of this warp's 16, lane 2i+1 the matching up feature
                 const uint32_t fl = q * 16u + (lane >> 1);
@@ -498,12 +419,7 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 if (PAIR == 2) mbar_arrive_cluster(empty_leader + as * 8u);
                 else mbar_arrive(empty_leader + as * 8u);
             }
-            if (PROF) busy += clock64() - t1;
             n_item += 1;
-        }
-        if (PROF && a.prof != NULL && warp == 2 && lane == 0) {
-            a.prof[blockIdx.x * 16u + 4u] = (unsigned long long)wait_acc;
-            a.prof[blockIdx.x * 16u + 5u] = (unsigned long long)busy;
         }
     }
     tc_fence_before();
@@ -514,7 +430,6 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (PAIR == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
-    if (PROF && a.prof != NULL && threadIdx.x == 0) a.prof[blockIdx.x * 16u] = (unsigned long long)(clock64() - t_begin);
 }
 
 // The chunk list as a kernel of its own (expert-parallel layer: the counts come from the plan): one block, thread =
@@ -526,27 +441,11 @@ moe_chunk_kernel(const uint32_t *__restrict__ count, const uint32_t *__restrict_
     moe_chunk_body(count, off, experts, chunks, n_chunks, max_chunks);
 }
 
-#ifdef MOE_WS_PROF
-__device__ unsigned long long g_ws_prof[256 * 16];
-__device__ unsigned long long g_ws_trace[2 * WS_TRACE_STEPS * 8];
-#endif
-
 template <int MODE, int PAIR>
-void ws_launch(moe_cuda_ctx *c, const CUtensorMap *tmW, const XMaps &tmX, WsArgs &a, uint32_t grid) {
-#ifdef MOE_WS_PROF
-    constexpr bool PROF = true;
-    MOE_CUDA_TRY(c, cudaGetSymbolAddress((void **)&a.prof, g_ws_prof));
-    MOE_CUDA_TRY(c, cudaGetSymbolAddress((void **)&a.trace, g_ws_trace));
-    const char *dbg = getenv("MOE_WS_DBG");
-    a.dbg = dbg != NULL ? (uint32_t)atoi(dbg) : 0u;
-    const char *only = getenv("MOE_WS_PROF_MODE");  // counters of one product only (1: gate_up, 2: down)
-    if (only != NULL && atoi(only) != MODE) a.prof = NULL;
-#else
-    constexpr bool PROF = false;
-#endif
+void ws_launch(moe_cuda_ctx *c, const CUtensorMap &tmW, const moe_xmaps &tmX, WsArgs &a, uint32_t grid) {
     int slot = MODE * 2 + (PAIR - 1);
     if (!c->sw_attr_set[slot]) {
-        MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_mm_ws_kernel<MODE, PAIR, PROF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_mm_ws_kernel<MODE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)ws_smem<PAIR>()));
         c->sw_attr_set[slot] = true;
     }
@@ -562,20 +461,11 @@ void ws_launch(moe_cuda_ctx *c, const CUtensorMap *tmW, const XMaps &tmX, WsArgs
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MOE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, moe_mm_ws_kernel<MODE, PAIR, PROF>, *tmW, tmX, a));
+    MOE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, moe_mm_ws_kernel<MODE, PAIR>, tmW, tmX, a));
     c->launches += 1;
 }
 
 }  // namespace
-
-#ifdef MOE_WS_PROF
-extern "C" void moe_ws_prof_read(unsigned long long *out, int words) {
-    cudaMemcpyFromSymbol(out, g_ws_prof, (size_t)words * 8);
-}
-extern "C" void moe_ws_trace_read(unsigned long long *out, int words) {
-    cudaMemcpyFromSymbol(out, g_ws_trace, (size_t)words * 8);
-}
-#endif
 
 void moe_launch_chunks(moe_cuda_ctx *c, const uint32_t *count, const uint32_t *off, uint32_t experts, void *chunks,
                        uint32_t *n_chunks, uint32_t max_chunks) {
@@ -596,30 +486,11 @@ void moe_launch_mm_ws(moe_cuda_ctx *c, int mode, int pair, const void *X, uint32
     MOE_REQUIRE(c, k % 8u == 0 && k >= 8u && rows_x >= 1, "mm_ws: k %u", k);
     MOE_REQUIRE(c, (uint64_t)experts_in_W * n < (1ull << 31), "mm_ws: expert count");
     MOE_REQUIRE(c, ((uintptr_t)C & 15) == 0 && (mode == MOE_MM_F32 || ldc % 8u == 0), "mm_ws: C not 16-byte addressable");
-    const CUtensorMap *tmW = mode == MOE_MM_SWIGLU_F16 ? moe_tmap_gate_up_f16(c, W, experts_in_W, n / 2u, k)
-                                                       : moe_tmap_2d_f16(c, W, (uint64_t)experts_in_W * n, k, 128, BK);
-    if (tmW == NULL) return;
-    XMaps tmX;
-    for (uint32_t i = 0; i < 8; i += 1) {
-        const CUtensorMap *m = moe_tmap_2d_f16(c, X, rows_x, k, 16u * (i + 1u), BK);
-        if (m == NULL) return;
-        tmX.m[i] = *m;
-    }
-#ifdef MOE_WS_PROF
-    {
-        cuuint64_t dims[2] = {256, (cuuint64_t)experts_in_W * n * k * 2 / 512};
-        cuuint64_t strides[1] = {512};
-        cuuint32_t box[2] = {256, 32};
-        cuuint32_t estr[2] = {1, 1};
-        typedef CUresult (*enc_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-        CUresult r = ((enc_fn)c->encode_tiled)(&tmX.wc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)W, dims, strides, box, estr,
-                                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        MOE_REQUIRE(c, r == CUDA_SUCCESS, "mm_ws: contiguous weight map failed: %d", (int)r);
-    }
-#endif
+    CUtensorMap tmW;
+    if (mode == MOE_MM_SWIGLU_F16 ? !moe_tmap_gate_up_f16(c, &tmW, W, experts_in_W, n / 2u, k)
+                                  : !moe_tmap_2d_f16(c, &tmW, W, (uint64_t)experts_in_W * n, k, 128)) return;
+    moe_xmaps tmX;
+    if (!moe_tmap_tokens_f16(c, &tmX, X, rows_x, k)) return;
     WsArgs a;
     a.C = C;
     a.chunks = (const uint4 *)chunks;
@@ -629,9 +500,6 @@ void moe_launch_mm_ws(moe_cuda_ctx *c, int mode, int pair, const void *X, uint32
     a.ldc = ldc;
     a.status = c->dev_status_dev;
     a.wait_ns = c->wait_ns;
-    a.prof = NULL;
-    a.trace = NULL;
-    a.dbg = 0;
     uint32_t ft = mode == MOE_MM_SWIGLU_F16 ? (n / 2u) / (64u * (uint32_t)pair) : n / (128u * (uint32_t)pair);
     uint64_t total = (uint64_t)max_chunks * ft * (uint32_t)pair;
     uint32_t sms = (uint32_t)c->sm_count / (uint32_t)pair * (uint32_t)pair;

@@ -123,10 +123,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// The same for a 64-byte swizzle (rows of 32 fp16): 8-row groups 512 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)(512u >> 4) << 32) | (1ull << 46) | (4ull << 61);
-}
 // Instruction descriptor, kind::f16: D fp32, A/B fp16, both K-major.
 __device__ __forceinline__ uint32_t umma_idesc(uint32_t m, uint32_t n) {
     return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);

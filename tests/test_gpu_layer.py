@@ -159,3 +159,22 @@ def test_upstream_projection_on_gpu_then_layer(ctx, mc, synth, oracle):
     assert np.array_equal(d_slot.read(np.uint32, (T, cfg.K)), ref.slot)
     h = d_h.read(np.float32, (T, 1, d))
     assert np.all(np.abs(h - ref.h) <= ATOL_OUT + RTOL_OUT * np.abs(ref.h))
+
+
+def test_many_tensor_maps_in_one_context(ctx, mc, synth, oracle):
+    """More operand buffers than a context keeps tensor maps for: the maps of a launch stay those of its own operands."""
+    import dataclasses
+    cfg = dataclasses.replace(synth.CONFIGS["c0"], T=200, name="c0-T200")
+    inp = synth.layer_inputs(cfg, 5)
+    ref = oracle.layer(inp.proj, inp.x16, inp.wgu, inp.wdown, cfg.K)
+    first = run_layer(ctx, mc, cfg, inp)
+    check(first, ref)
+    n = 700
+    a, w, out = ctx.zeros((n + 1) * 16 * 64), ctx.zeros(128 * 8 * 2), ctx.alloc(8 * 128 * 4)
+    for i in range(n):
+        ctx.dense(a.ptr + i * 16 * 64, w, out, None, 8, 128, 8)
+    small = dataclasses.replace(cfg, T=72, name="c0-T72")
+    part = synth.layer_inputs(small, 5)
+    check(run_layer(ctx, mc, small, part), oracle.layer(part.proj, part.x16, part.wgu, part.wdown, cfg.K))
+    again = run_layer(ctx, mc, cfg, inp)
+    assert np.array_equal(again["h"], first["h"])
