@@ -267,6 +267,32 @@ def test_kd_bytes(ctx, oracle):
         assert differ.mean() < 0.01
 
 
+@pytest.mark.parametrize("rows,vocab,alphabet,lift", [
+    (1, 1, 4, 0.0), (3, 1023, 4, 0.0), (33, 1025, 2, 0.0), (32, 4096, 1, 0.0), (65, 2049, 26, 130.0), (7, 5000, 250, -130.0)])
+def test_kd_bytes_edges(ctx, oracle, rows, vocab, alphabet, lift):
+    """Edges of the 1024-token chunks and 32-row groups; all tokens behind the same bytes (alphabet 1); a row maximum
+    that a later chunk exceeds by more than the reference may lag (lift added to the last 600 logits)."""
+    rng = np.random.default_rng(vocab)
+    length = rng.integers(0, 17, vocab)
+    tb = rng.integers(3, 3 + alphabet, (vocab, 16)).astype(np.uint8)
+    tb[np.arange(16)[None, :] >= length[:, None]] = 0
+    toks = np.ascontiguousarray(np.concatenate([tb.view(np.uint32).reshape(vocab, 4), length[:, None].astype(np.uint32)], 1))
+    cont = np.zeros((rows, 5), np.uint32)
+    cont[:, :4] = rng.integers(3, 3 + alphabet, (rows, 16)).astype(np.uint8).view(np.uint32).reshape(rows, 4)
+    cont[:, 4] = [16, 1, 2, 3, 0, 40][:rows] if rows <= 6 else rng.integers(0, 18, rows)
+    logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
+    logits[:, -600:] += np.float32(lift)
+    d_out = ctx.alloc(rows * 16 * 8 * 4).fill(0xdeadbeef)
+    ctx.kd_bytes(ctx.upload(logits), ctx.upload(toks), ctx.upload(cont), d_out, rows, vocab)
+    ctx.flush()
+    got, ref = d_out.read(np.uint32, (rows, 16, 8)), oracle.kd_bytes(logits, toks, cont)
+    pg = (got >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    pr = (ref >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    assert np.all(np.abs(pg - pr) <= 1.5e-3 * pr + 1e-7)   # half a unit of the fp16 result, and fp32 sums in another order
+    assert np.array_equal(got[..., 0] & 0xffff, ref[..., 0] & 0xffff)
+    assert ((got & 0xffff) != (ref & 0xffff)).mean() < 0.01
+
+
 def test_fill_and_copy(ctx):
     b = ctx.alloc(4 * 1003)
     b.fill(0x12345678)
