@@ -16,7 +16,7 @@
 #define MOE_TILE 128u         // MDA_QWEN_TILE, src/qwen.h:14
 
 // Scratch areas inside the context (grown on demand, never shrunk).
-enum { MOE_SCR_SCATTER = 0, MOE_SCR_LAYER = 1, MOE_SCR_STAGE = 2, MOE_SCR_EP = 3, MOE_SCR_COUNT = 4 };
+enum { MOE_SCR_SCATTER = 0, MOE_SCR_LAYER = 1, MOE_SCR_STAGE = 2, MOE_SCR_EP = 3, MOE_SCR_KD = 4, MOE_SCR_COUNT = 5 };
 
 // Tensor maps already made, by what they describe: a hash picks a set of MOE_TMAP_WAYS entries, a full set gives up its
 // entries in turn.  512 entries hold the weights of a 48-layer stack (3 per layer) beside everything else of a context;

@@ -205,7 +205,7 @@ __device__ __forceinline__ uint32_t kd_slot(uint32_t idx) { return (idx & ~127u)
 template <bool VEC>  // rows can be read 16 bytes at a time
 __global__ void __launch_bounds__(KD_THREADS, 2)
 moe_kd_mass_kernel(const float *__restrict__ logits, const uint32_t *__restrict__ sorted, const uint32_t *__restrict__ cont,
-                   const uint32_t *__restrict__ row_map, float *bins, float *__restrict__ part, float2 *__restrict__ refs, uint32_t vocab, uint32_t rows, uint32_t splits) {
+                   const uint32_t *__restrict__ row_map, float *bins, float2 *__restrict__ refs, uint32_t vocab, uint32_t rows, uint32_t splits) {
     extern __shared__ __align__(16) uint8_t kd_raw[];
     kd_mass_smem &sm = *reinterpret_cast<kd_mass_smem *>(kd_raw);
     const uint32_t lid = threadIdx.x, lane = lid & 31u, warp = lid >> 5;
@@ -369,8 +369,7 @@ moe_kd_mass_kernel(const float *__restrict__ logits, const uint32_t *__restrict_
     // the bins turned to [row][bin] for the kernel that puts a row together
     for (uint32_t i = lid; i < KD_BINS * KD_ROWS; i += KD_THREADS) sm.tile[(i / KD_ROWS) * KD_PITCH + i % KD_ROWS] = __ldcg(bins + i);
     __syncthreads();
-    part += (size_t)blockIdx.x * KD_BINS * KD_ROWS;
-    for (uint32_t i = lid; i < KD_BINS * KD_ROWS; i += KD_THREADS) part[i] = sm.tile[(i % KD_BINS) * KD_PITCH + i / KD_BINS];
+    for (uint32_t i = lid; i < KD_BINS * KD_ROWS; i += KD_THREADS) bins[i] = sm.tile[(i % KD_BINS) * KD_PITCH + i / KD_BINS];
 #pragma unroll
     for (uint32_t k = 0; k < KD_RPW; k += 1) {
         if (lane == 0) refs[(size_t)blockIdx.x * KD_ROWS + warp * KD_RPW + k] = make_float2(ref[k], top[k]);
@@ -380,7 +379,7 @@ moe_kd_mass_kernel(const float *__restrict__ logits, const uint32_t *__restrict_
 // One block per row.
 __global__ void __launch_bounds__(KD_RTHREADS, 3)
 moe_kd_rows_kernel(const float *__restrict__ logits, const uint4 *__restrict__ bytes, const uint32_t *__restrict__ sorted,
-                   const uint32_t *__restrict__ cont, const uint32_t *__restrict__ row_map, const float *__restrict__ part, const float2 *__restrict__ refs,
+                   const uint32_t *__restrict__ cont, const uint32_t *__restrict__ row_map, const float *__restrict__ bins, const float2 *__restrict__ refs,
                    uint32_t *__restrict__ outp, uint32_t vocab, uint32_t splits) {
     __shared__ float H[KD_D][256];
     __shared__ float H2[KD_RWARPS][256];  // depth 2, a copy per warp: its bins take most of the adds
@@ -421,7 +420,7 @@ moe_kd_rows_kernel(const float *__restrict__ logits, const uint4 *__restrict__ b
     m = s_max;
 #pragma unroll
     for (uint32_t b = lid; b < KD_BINS; b += KD_RTHREADS) {
-        const float *p = part + blk0 * KD_BINS + b;
+        const float *p = bins + blk0 * KD_BINS + b;
         float sum = 0.0f;
 #pragma unroll 8
         for (uint32_t s = 0; s < splits; s += 1) sum += p[(size_t)s * KD_ROWS * KD_BINS] * scale[s];
@@ -604,14 +603,13 @@ extern "C" void moe_cuda_kd_bytes(moe_cuda_ctx_t *c, const float *logits, const 
         }
     }
     const size_t blocks_max = (size_t)groups_max * splits, tokens = (size_t)n_chunks * KD_CHUNK;
-    const size_t part_bytes = blocks_max * KD_ROWS * KD_BINS * sizeof(float);
-    uint8_t *scr = (uint8_t *)moe_scratch(c, MOE_SCR_STAGE, tokens * (sizeof(uint4) + sizeof(uint32_t)) + 2u * part_bytes +
+    const size_t bins_bytes = blocks_max * KD_ROWS * KD_BINS * sizeof(float);
+    uint8_t *scr = (uint8_t *)moe_scratch(c, MOE_SCR_KD, tokens * (sizeof(uint4) + sizeof(uint32_t)) + bins_bytes +
                                                                 blocks_max * KD_ROWS * sizeof(float2) + (size_t)pc.rows * sizeof(uint32_t));
     if (scr == NULL) return;
     uint4 *bytes = (uint4 *)scr;
-    float *part = (float *)(bytes + tokens);
-    float *bins = part + part_bytes / sizeof(float);
-    float2 *refs = (float2 *)(bins + part_bytes / sizeof(float));
+    float *bins = (float *)(bytes + tokens);
+    float2 *refs = (float2 *)(bins + bins_bytes / sizeof(float));
     uint32_t *sorted = (uint32_t *)(refs + blocks_max * KD_ROWS);
     uint32_t *row_map = sorted + tokens;
     const bool vec = pc.vocab % 4u == 0 && ((uintptr_t)logits & 15) == 0;
@@ -625,10 +623,10 @@ extern "C" void moe_cuda_kd_bytes(moe_cuda_ctx_t *c, const float *logits, const 
     MOE_LAUNCHED(c);
     for (uint32_t row0 = 0; row0 < pc.rows; row0 += batch) {  // row_map holds rows of the whole call
         const uint32_t rows = pc.rows - row0 < batch ? pc.rows - row0 : batch, groups = (rows + KD_ROWS - 1u) / KD_ROWS;
-        if (vec) moe_kd_mass_kernel<true><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, part, refs, pc.vocab, rows, splits);
-        else moe_kd_mass_kernel<false><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, part, refs, pc.vocab, rows, splits);
+        if (vec) moe_kd_mass_kernel<true><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, refs, pc.vocab, rows, splits);
+        else moe_kd_mass_kernel<false><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, refs, pc.vocab, rows, splits);
         MOE_LAUNCHED(c);
-        moe_kd_rows_kernel<<<rows, KD_RTHREADS, 0, c->stream>>>(logits, bytes, sorted, cont, row_map + row0, part, refs, outp, pc.vocab, splits);
+        moe_kd_rows_kernel<<<rows, KD_RTHREADS, 0, c->stream>>>(logits, bytes, sorted, cont, row_map + row0, bins, refs, outp, pc.vocab, splits);
         MOE_LAUNCHED(c);
     }
 }
