@@ -216,6 +216,19 @@ extern "C" void moe_cuda_combine(moe_cuda_ctx_t *c, const float *wt, const uint3
 // ---- glue: shader/qwen_elem.comp op 0, shader/absmax.comp, shader/cast_f16.comp ----
 __device__ __forceinline__ float moe_silu(float v) { return v / (1.0f + expf(-v)); }  // qwen_elem.comp:16-18
 
+// These kernels are bound by HBM.  Four values per load and several independent loads per thread keep enough bytes in
+// flight; the scalar forms (one 4-byte load per thread and iteration, a 64-bit division per value in the SwiGLU) reached
+// 2.5 to 4 TB/s.  Measured for 24,320 x 768 SwiGLU outputs, absmax and cast of them: 90, 33 and 26 us scalar against
+// 37, 14 and 11 us; absmax and cast of 3001 x 8192: 48 and 42 against 19 and 19 us.
+#define EL_THREADS 256u
+#define EL_VECS 4u  // 16-byte loads per thread
+
+__device__ __forceinline__ float moe_elem(float g, float u, uint32_t op, float scale) {
+    return op == 0u ? __fmul_rn(moe_silu(g), u)    // qwen_elem.comp:27
+                    : moe_silu(__fmul_rn(g, scale));  // :29 (the mixer's gate, src/qwen.c:648-657)
+}
+
+// General form: any n, stride, offset and alignment.
 __global__ void moe_swiglu_kernel(const float *__restrict__ a, float *__restrict__ y, uint32_t rows, uint32_t n,
                                   uint32_t astride, uint32_t ao, uint32_t bo, uint32_t op, float scale) {
     size_t total = (size_t)rows * n;
@@ -223,9 +236,33 @@ __global__ void moe_swiglu_kernel(const float *__restrict__ a, float *__restrict
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         size_t r = i / n;
         uint32_t cidx = (uint32_t)(i - r * n);
-        float g = a[r * astride + ao + cidx];
-        if (op == 0u) y[i] = __fmul_rn(moe_silu(g), a[r * astride + bo + cidx]);  // qwen_elem.comp:27
-        else y[i] = moe_silu(__fmul_rn(g, scale));                                // :29 (the mixer's gate, src/qwen.c:648-657)
+        y[i] = moe_elem(a[r * astride + ao + cidx], op == 0u ? a[r * astride + bo + cidx] : 0.0f, op, scale);
+    }
+}
+
+// Rows, offsets and strides in whole float4: total4 = rows * n4 values of four, below 2^31.
+template <uint32_t OP>
+__global__ void __launch_bounds__(EL_THREADS)
+moe_swiglu4_kernel(const float4 *__restrict__ a, float4 *__restrict__ y, uint32_t total4, uint32_t n4, uint32_t astride4,
+                   uint32_t ao4, uint32_t bo4, float scale) {
+    constexpr uint32_t U = 2;  // two operands: four loads in flight
+    const uint32_t i0 = blockIdx.x * (EL_THREADS * U) + threadIdx.x;
+    float4 g[U], u[U];
+#pragma unroll
+    for (uint32_t j = 0; j < U; j += 1) {
+        const uint32_t i = i0 + j * EL_THREADS;
+        if (i >= total4) break;
+        const uint32_t r = i / n4;
+        const float4 *row = a + (size_t)r * astride4 + (i - r * n4);
+        g[j] = __ldg(row + ao4);
+        u[j] = OP == 0u ? __ldg(row + bo4) : g[j];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < U; j += 1) {
+        const uint32_t i = i0 + j * EL_THREADS;
+        if (i >= total4) break;
+        y[i] = make_float4(moe_elem(g[j].x, u[j].x, OP, scale), moe_elem(g[j].y, u[j].y, OP, scale),
+                           moe_elem(g[j].z, u[j].z, OP, scale), moe_elem(g[j].w, u[j].w, OP, scale));
     }
 }
 
@@ -235,24 +272,53 @@ extern "C" void moe_cuda_swiglu(moe_cuda_ctx_t *c, const float *a, float *y, str
     MOE_REQUIRE(c, a != NULL && y != NULL, "swiglu: null buffer");
     size_t total = (size_t)pc.rows * pc.n;
     if (total == 0) return;
+    // four values at a time where every row starts on 16 bytes; index arithmetic of 32 bits up to 2^33 values
+    if (((uintptr_t)a | (uintptr_t)y) % 16 == 0 && (pc.n | pc.astride | pc.ao | (pc.op == 0u ? pc.bo : 0u)) % 4u == 0 &&
+        total / 4 < (1ull << 31)) {
+        const uint32_t total4 = (uint32_t)(total / 4), blocks = (total4 + 2u * EL_THREADS - 1u) / (2u * EL_THREADS);
+        if (pc.op == 0u)
+            moe_swiglu4_kernel<0><<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)a, (float4 *)y, total4, pc.n / 4u,
+                                                                       pc.astride / 4u, pc.ao / 4u, pc.bo / 4u, pc.scale);
+        else
+            moe_swiglu4_kernel<1><<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)a, (float4 *)y, total4, pc.n / 4u,
+                                                                       pc.astride / 4u, pc.ao / 4u, 0, pc.scale);
+        MOE_LAUNCHED(c);
+        return;
+    }
     size_t blocks = (total + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
     moe_swiglu_kernel<<<(unsigned)blocks, 256, 0, c->stream>>>(a, y, pc.rows, pc.n, pc.astride, pc.ao, pc.bo, pc.op, pc.scale);
     MOE_LAUNCHED(c);
 }
 
-__global__ void __launch_bounds__(256)
-moe_absmax_kernel(const float *__restrict__ x, uint32_t *__restrict__ amax, size_t n, uint32_t slot) {
-    __shared__ float red[8];
-    size_t stride = (size_t)gridDim.x * blockDim.x;
+// n4 float4 from the first 16-byte boundary of x on; the few values before and behind them go to the first threads.
+__global__ void __launch_bounds__(EL_THREADS)
+moe_absmax_kernel(const float *__restrict__ x, uint32_t *__restrict__ amax, uint32_t n, uint32_t head, uint32_t slot) {
+    __shared__ float red[EL_THREADS / 32];
+    const uint32_t n4 = (n - head) / 4u, stride = gridDim.x * EL_THREADS;
+    const float4 *x4 = reinterpret_cast<const float4 *>(x + head);
+    const uint32_t first = blockIdx.x * EL_THREADS + threadIdx.x;
     float m = 0.0f;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) m = fmaxf(m, fabsf(x[i]));
+    for (uint32_t base = first; base < n4; base += EL_VECS * stride) {
+        float4 v[EL_VECS];
+#pragma unroll
+        for (uint32_t j = 0; j < EL_VECS; j += 1) {
+            v[j] = base + j * stride < n4 ? __ldg(x4 + base + j * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < EL_VECS; j += 1) {
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+        }
+    }
+    if (first < head) m = fmaxf(m, fabsf(x[first]));
+    const uint32_t tail = head + 4u * n4 + first;
+    if (first < 4u && tail < n) m = fmaxf(m, fabsf(x[tail]));
 #pragma unroll
     for (uint32_t o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; w += 1) m = fmaxf(m, red[w]);
+        for (uint32_t w = 1; w < EL_THREADS / 32; w += 1) m = fmaxf(m, red[w]);
         atomicMax(&amax[slot], __float_as_uint(m));  // absmax.comp:29; valid for non-negative floats
     }
 }
@@ -261,12 +327,20 @@ extern "C" void moe_cuda_absmax(moe_cuda_ctx_t *c, const float *x, uint32_t *ama
     if (!MOE_LIVE(c)) return;
     MOE_REQUIRE(c, x != NULL && amax != NULL && pc.slot != MDA_PC_NO_SLOT, "absmax: null buffer or no slot");
     if (pc.n == 0) return;
-    uint32_t blocks = (pc.n + 255u) / 256u;
+    uint32_t head = (uint32_t)((16u - (uintptr_t)x % 16u) % 16u / 4u);
+    if (head > pc.n) head = pc.n;
+    uint32_t blocks = (uint32_t)(((uint64_t)pc.n + 4u * EL_VECS * EL_THREADS - 1u) / (4u * EL_VECS * EL_THREADS));
     if (blocks > (uint32_t)c->sm_count * 8u) blocks = (uint32_t)c->sm_count * 8u;
-    moe_absmax_kernel<<<blocks, 256, 0, c->stream>>>(x, amax, pc.n, pc.slot);
+    moe_absmax_kernel<<<blocks, EL_THREADS, 0, c->stream>>>(x, amax, pc.n, head, pc.slot);
     MOE_LAUNCHED(c);
 }
 
+__device__ __forceinline__ uint2 moe_pack4(float4 v, float s) {
+    __half2 lo = __floats2half2_rn(v.x * s, v.y * s), hi = __floats2half2_rn(v.z * s, v.w * s);  // cast_f16.comp:33
+    return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+}
+
+// General form: any alignment.
 __global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__restrict__ dst, size_t n,
                                     const uint32_t *__restrict__ amax, uint32_t slot) {
     float s = moe_slot_scale(amax, slot);
@@ -276,12 +350,37 @@ __global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__res
     }
 }
 
+// src on 16 bytes, dst on 8.
+__global__ void __launch_bounds__(EL_THREADS)
+moe_cast4_f16_kernel(const float4 *__restrict__ src, uint2 *__restrict__ dst, uint32_t n, const uint32_t *__restrict__ amax,
+                     uint32_t slot) {
+    const uint32_t n4 = n / 4u, i0 = blockIdx.x * (EL_THREADS * EL_VECS) + threadIdx.x;
+    float4 v[EL_VECS];
+#pragma unroll
+    for (uint32_t j = 0; j < EL_VECS; j += 1) {
+        if (i0 + j * EL_THREADS < n4) v[j] = __ldg(src + i0 + j * EL_THREADS);
+    }
+    const float s = moe_slot_scale(amax, slot);
+#pragma unroll
+    for (uint32_t j = 0; j < EL_VECS; j += 1) {
+        if (i0 + j * EL_THREADS < n4) dst[i0 + j * EL_THREADS] = moe_pack4(v[j], s);
+    }
+    const uint32_t tail = 4u * n4 + i0;
+    if (i0 < 4u && tail < n) reinterpret_cast<__half *>(dst)[tail] = __float2half_rn(reinterpret_cast<const float *>(src)[tail] * s);
+}
+
 extern "C" void moe_cuda_cast_f16(moe_cuda_ctx_t *c, const float *src, void *dst, const uint32_t *amax,
                                   struct mda_pc_cast_t pc) {
     if (!MOE_LIVE(c)) return;
     MOE_REQUIRE(c, src != NULL && dst != NULL && (amax != NULL || pc.slot == MDA_PC_NO_SLOT), "cast: null buffer");
     if (pc.n == 0) return;
-    uint32_t blocks = (pc.n + 255u) / 256u;
+    if ((uintptr_t)src % 16 == 0 && (uintptr_t)dst % 8 == 0) {
+        const uint32_t per = 4u * EL_VECS * EL_THREADS, blocks = (uint32_t)(((uint64_t)pc.n + per - 1u) / per);
+        moe_cast4_f16_kernel<<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)src, (uint2 *)dst, pc.n, amax, pc.slot);
+        MOE_LAUNCHED(c);
+        return;
+    }
+    uint32_t blocks = (uint32_t)(((uint64_t)pc.n + 255u) / 256u);
     if (blocks > (uint32_t)c->sm_count * 16u) blocks = (uint32_t)c->sm_count * 16u;
     moe_cast_f16_kernel<<<blocks, 256, 0, c->stream>>>(src, (__half *)dst, pc.n, amax, pc.slot);
     MOE_LAUNCHED(c);

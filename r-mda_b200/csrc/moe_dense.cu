@@ -81,12 +81,46 @@ __global__ void moe_hc_kernel(const float *__restrict__ a, const float *__restri
     }
 }
 
+// The read-out with four columns per thread (d % 4 == 0, 16-byte aligned): all 2 * HC loads of a thread are in flight
+// together.  Bound by HBM; 3001 rows of 4 x 2048: 76 us one column at a time, 35 us this way.
+template <uint32_t HC>
+__global__ void __launch_bounds__(NR_THREADS)
+moe_hc_read4_kernel(const float4 *__restrict__ a, const float4 *__restrict__ b, float4 *__restrict__ h, uint32_t total4, uint32_t d4) {
+    const uint32_t i = blockIdx.x * NR_THREADS + threadIdx.x;
+    if (i >= total4) return;
+    const uint32_t r = i / d4;
+    const size_t j0 = (size_t)r * HC * d4 + (i - r * d4);
+    float4 av[HC], bv[HC];
+#pragma unroll
+    for (uint32_t s = 0; s < HC; s += 1) {
+        av[s] = __ldg(a + j0 + (size_t)s * d4);
+        bv[s] = __ldg(b + j0 + (size_t)s * d4);
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (uint32_t s = 0; s < HC; s += 1) {
+        acc.x += dn_sigmoid(av[s].x) * bv[s].x;
+        acc.y += dn_sigmoid(av[s].y) * bv[s].y;
+        acc.z += dn_sigmoid(av[s].z) * bv[s].z;
+        acc.w += dn_sigmoid(av[s].w) * bv[s].w;
+    }
+    h[i] = make_float4(acc.x / (float)HC, acc.y / (float)HC, acc.z / (float)HC, acc.w / (float)HC);
+}
+
 extern "C" void moe_cuda_hc(moe_cuda_ctx_t *c, const float *a, const float *b, float *h, struct mda_pc_qwen_hc_t pc) {
     if (!MOE_LIVE(c)) return;
     MOE_REQUIRE(c, pc.op <= 2u && pc.hc >= 1 && pc.d >= 1, "hc: bad op or shape");
     MOE_REQUIRE(c, a != NULL && b != NULL && h != NULL, "hc: null buffer");
     const size_t n = (size_t)pc.rows * pc.d * (pc.op == 2u ? pc.hc : 1u);
     if (n == 0) return;
+    // the teacher's four streams; other counts and ragged or unaligned rows take the general form below
+    if (pc.op == 0u && pc.hc == 4u && pc.d % 4u == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)h) % 16 == 0 && n / 4 < (1ull << 31)) {
+        const uint32_t total4 = (uint32_t)(n / 4);
+        moe_hc_read4_kernel<4><<<(total4 + NR_THREADS - 1u) / NR_THREADS, NR_THREADS, 0, c->stream>>>(
+            (const float4 *)a, (const float4 *)b, (float4 *)h, total4, pc.d / 4u);
+        MOE_LAUNCHED(c);
+        return;
+    }
     size_t blocks = (n + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
     moe_hc_kernel<<<(unsigned)blocks, 256, 0, c->stream>>>(a, b, h, pc);

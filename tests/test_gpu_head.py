@@ -29,8 +29,17 @@ def test_norm(ctx, oracle, rows, groups, gsize, op):
 
 @pytest.mark.parametrize("op", [0, 1, 2])
 def test_hc(ctx, oracle, op):
+    _check_hc(ctx, oracle, op, 50, 192, 4)
+
+
+@pytest.mark.parametrize("rows,d,hc", [(1, 4, 4), (7, 1028, 4), (3, 190, 4), (9, 256, 3)])
+def test_hc_read_out_widths(ctx, oracle, rows, d, hc):
+    _check_hc(ctx, oracle, 0, rows, d, hc)
+
+
+def _check_hc(ctx, oracle, op, rows, d, hc):
     rng = np.random.default_rng(op)
-    rows, d, hc, stride, off = 50, 192, 4, 24, 17
+    stride, off = 24, 17
     if op == 0:
         a, b = rng.standard_normal((rows, hc * d)).astype(np.float32), rng.standard_normal((rows, hc * d)).astype(np.float32)
         h0 = np.full((rows, d), np.nan, np.float32)

@@ -229,6 +229,39 @@ def test_glue(ctx, oracle, mc):
     assert 16384 <= np.abs(ref16.view(np.float16).astype(np.float32)).max() < 32768  # shader/cast_f16.comp scale
 
 
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,n,astride,ao,bo", [(1, 1, 2, 0, 1), (3, 5, 12, 1, 7), (2, 4, 8, 0, 4), (5, 260, 1024, 4, 512),
+                                                  (129, 1028, 2056, 0, 1028), (7, 2047, 4096, 0, 2047)])
+def test_glue_edges(ctx, oracle, rows, n, astride, ao, bo, shift):
+    """Value counts, strides and buffers (`shift` floats off 16 bytes) on both sides of the four-at-a-time forms."""
+    rng = np.random.default_rng(rows * n + shift)
+    a = (rng.standard_normal((rows, astride)) * 3).astype(np.float32)
+    pad = np.full(shift, 1e9, np.float32)   # in front of the values: a read too early changes the maximum
+    d_a, d_hp = ctx.upload(np.concatenate([pad, a.ravel(), pad])), ctx.upload(np.full(rows * n + 8, 1e9, np.float32))
+    hp_at = d_hp.ptr + 4 * shift
+    ctx.swiglu(d_a.ptr + 4 * shift, hp_at, rows, n, astride, ao, bo)
+    ctx.flush()
+    raw = d_hp.read(np.float32, (rows * n + 8,))
+    hp = raw[shift:shift + rows * n].reshape(rows, n).copy()
+    assert np.allclose(hp, oracle.swiglu(a, n, astride, ao, bo), rtol=2e-6, atol=1e-7)
+    assert np.all(raw[:shift] == 1e9) and np.all(raw[shift + rows * n:] == 1e9)
+    hp[-1, -1] = -77.0   # the largest value last, then not a number in front of it
+    for first in (1.0, np.nan):
+        hp[0, 0] = first if hp.size > 1 else -77.0
+        d_v = ctx.upload(np.concatenate([pad, hp.ravel(), np.full(4, 1e9, np.float32)]))
+        amax = oracle.absmax(np.nan_to_num(hp), np.zeros(4, np.uint32), 1)
+        d_amax = ctx.zeros(16)
+        ctx.absmax(d_v.ptr + 4 * shift, d_amax, rows * n, 1)
+        d_16 = ctx.upload(np.full(rows * n + 8, 0xabcd, np.uint16))
+        ctx.cast_f16(d_v.ptr + 4 * shift, d_16.ptr + 2 * shift, d_amax, rows * n, 1)
+        ctx.flush()
+        assert np.array_equal(d_amax.read(np.uint32, (4,)), amax)
+        got = d_16.read(np.uint16, (rows * n + 8,))
+        ref, mine = oracle.cast_f16(hp, amax, 1).view(np.float16), got[shift:shift + rows * n].reshape(rows, n).view(np.float16)
+        assert np.array_equal(mine, ref, equal_nan=True)
+        assert np.all(got[:shift] == 0xabcd) and np.all(got[shift + rows * n:] == 0xabcd)
+
+
 def test_bf16_to_f16_in_place(ctx, oracle):
     """The weight-upload conversion (shader/qwen_bf16.comp): bit-exact, odd word counts, specials."""
     rng = np.random.default_rng(8)
