@@ -140,13 +140,12 @@ enum { MOE_MM_F32 = 0, MOE_MM_SWIGLU_F16 = 1, MOE_MM_F16 = 2 };
 // Grouped product.  mode F32: C fp32 [m x n] = A*B^T * s;  SWIGLU_F16: B holds
 // [gate n/2 rows | up n/2 rows] per expert and C fp16 [m x n/2] = silu(gate)*up;
 // F16: C fp16 [m x n].
-// a_rows = rows A really holds (<= m); rows beyond read as zero.  c_rows (fp32 mode; 0 = m) = rows C really
-// holds; rows beyond are not stored.  With src_row (SWIGLU_F16 only)
+// a_rows = rows A really holds (<= m); rows beyond read as zero.  With src_row (SWIGLU_F16 only)
 // A is the un-permuted activation matrix [a_rows x k] and tile row p is its row src_row[p].
 void moe_launch_mm(moe_cuda_ctx *c, int mode, const void *A, const void *B, void *C,
                    const uint32_t *amax, const uint32_t *tiles, uint32_t m, uint32_t n, uint32_t k,
                    uint32_t sa, uint32_t sb, uint32_t experts_in_B, uint32_t a_rows, bool prefix = false,
-                   const uint32_t *src_row = NULL, uint32_t c_rows = 0);
+                   const uint32_t *src_row = NULL);
 
 // Weight-stationary grouped product over token chunks (moe_mm_ws.cu).
 void moe_launch_chunks(moe_cuda_ctx *c, const uint32_t *count, const uint32_t *off, uint32_t experts, void *chunks,
@@ -154,6 +153,10 @@ void moe_launch_chunks(moe_cuda_ctx *c, const uint32_t *count, const uint32_t *o
 void moe_launch_mm_ws(moe_cuda_ctx *c, int mode, int pair, const void *X, uint32_t rows_x, const void *W,
                         uint32_t experts_in_W, void *C, uint32_t ldc, const void *chunks, const uint32_t *n_chunks,
                         uint32_t max_chunks, uint32_t n, uint32_t k);
+
+// The same kernel over all rows (moe_cuda_dense; small moe_cuda_mm calls with their tile schedule).
+void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C, const uint32_t *amax, const uint32_t *tiles,
+                         uint32_t rows, uint32_t n, uint32_t k, uint32_t sa, uint32_t sb, uint32_t experts_in_W);
 
 struct moe_combine_args {
     const float *wt;

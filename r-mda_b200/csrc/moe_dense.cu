@@ -5,8 +5,8 @@
 //   moe_cuda_norm    shader/qwen_norm.comp op 0 / op 1 (grouped RMSNorm)
 //   moe_cuda_hc      shader/qwen_hc.comp ops 0, 1, 2
 //   moe_cuda_dense   C[rows x n] fp32 = A16[rows x k] * W[n x k]^T / scale(sa):
-//                    the grouped tcgen05 kernel of moe_mm.cu over a dense tile
-//                    schedule (one "expert", every 128-row tile used)
+//                    the weight-stationary tcgen05 kernel of moe_mm_ws.cu over
+//                    all rows (one "expert")
 // Elementwise kernels are HBM bound: 128-bit accesses, coalesced along the row.
 #include "moe_common.cuh"
 
@@ -136,10 +136,5 @@ extern "C" void moe_cuda_dense(moe_cuda_ctx_t *c, const void *A16, const void *W
     MOE_REQUIRE(c, A16 != NULL && W != NULL && C != NULL, "dense: null buffer");
     MOE_REQUIRE(c, pc.rows >= 1 && pc.n % 128u == 0 && pc.n >= 128u && pc.k % 8u == 0 && pc.k >= 8u,
                 "dense: rows %u n %u k %u (n must be a multiple of 128, k of 8)", pc.rows, pc.n, pc.k);
-    const uint32_t m = (pc.rows + MOE_TILE - 1u) / MOE_TILE * MOE_TILE;
-    // the dense tile schedule: every 128-row tile belongs to "expert" 0
-    uint32_t *tiles = (uint32_t *)moe_scratch(c, MOE_SCR_STAGE, (size_t)(m / MOE_TILE) * 4);
-    if (tiles == NULL) return;
-    MOE_CUDA_TRY(c, cudaMemsetAsync(tiles, 0, (size_t)(m / MOE_TILE) * 4, c->stream));
-    moe_launch_mm(c, MOE_MM_F32, A16, W, C, amax, tiles, m, pc.n, pc.k, pc.sa, MDA_PC_NO_SLOT, 1, pc.rows, true, NULL, pc.rows);
+    moe_launch_mm_dense(c, A16, W, C, amax, NULL, pc.rows, pc.n, pc.k, pc.sa, MDA_PC_NO_SLOT, 1);
 }

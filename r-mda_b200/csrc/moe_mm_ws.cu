@@ -33,7 +33,8 @@ constexpr uint32_t NPROD = 3;               // issuing threads per operand, taki
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ET = 32;                  // tokens per epilogue step (one tcgen05.ld of 32 columns)
 constexpr uint32_t PITCH_SW = 160;           // bytes per token row of the turn-round tile, SwiGLU (64 fp16 + pad)
-constexpr uint32_t PITCH_F16 = 256;          // the same for 128 fp16 features
+constexpr uint32_t PITCH_F16 = 256;          // pitch of the two turn-round buffers
+constexpr uint32_t PITCH_T = 80;             // bytes per token row of a warp's own tile of 32 fp16 features: eight rows meet eight bank groups
 constexpr uint32_t TURN_BYTES = 2 * ET * PITCH_F16;  // two buffers
 
 template <int PAIR>
@@ -66,7 +67,16 @@ struct WsArgs {
     uint32_t ldc;              // row stride of C in elements
     uint32_t *status;
     uint64_t wait_ns;
+    // dense form (MM_DENSE): no chunk list, rows are cut into chunks of `per` (a multiple of 16)
+    uint32_t rows, per;
+    uint32_t splits, ksplit;   // K split `splits` ways, ksplit K steps each; split p of C starts at C + p * rows * ldc
+    const uint32_t *tiles;     // or NULL: expert of each 128-row tile, >= experts: the tile is skipped (per divides 128)
+    uint32_t experts;
+    const uint32_t *amax;      // scale slots (power of two) of both operands
+    uint32_t sa, sb;
 };
+// C fp32 = X * W^T over all rows, for moe_cuda_dense and small moe_cuda_mm calls
+constexpr int MM_DENSE = 3;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -78,8 +88,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
 }
+// Relaxed: a release at cluster scope waits until the warp's global stores have been performed (3100 cycles per item of
+// the down product).  What the barrier hands over is the accumulator, whose reads are complete (tcgen05.wait::ld) and
+// ordered by tcgen05.fence::before_thread_sync.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -158,10 +171,29 @@ __device__ __forceinline__ uint32_t x_rows_loaded(uint32_t half) {
     return rows;
 }
 struct WsItem {
-    uint32_t e, row0, ntok, nvalid, ft;
+    uint32_t e, row0, ntok, nvalid, ft, kb0, kb1, split;
 };
 
-__device__ __forceinline__ void ws_item(const WsArgs &a, uint32_t w, uint32_t ft_count, WsItem &it) {
+// False: nothing to do for this item (dense form: an unused row tile).
+template <int MODE>
+__device__ __forceinline__ bool ws_item(const WsArgs &a, uint32_t w, uint32_t ft_count, uint32_t kblocks, WsItem &it) {
+    if (MODE == MM_DENSE) {
+        // splits, then chunks, then feature tiles: CTAs that run together share weight tiles, so that a weight
+        // matrix larger than L2 (a vocabulary) comes from HBM once
+        const uint32_t nch = (a.rows + a.per - 1u) / a.per;
+        const uint32_t q = w / a.splits;
+        it.split = w - q * a.splits;
+        it.ft = q / nch;
+        it.row0 = (q - it.ft * nch) * a.per;
+        it.nvalid = min(a.per, a.rows - it.row0);
+        it.ntok = (it.nvalid + 15u) & ~15u;
+        it.kb0 = it.split * a.ksplit;
+        it.kb1 = min(it.kb0 + a.ksplit, kblocks);
+        it.e = a.tiles != NULL ? a.tiles[it.row0 / MOE_TILE] : 0u;
+        return it.e < a.experts;
+    }
+    it.kb0 = 0;
+    it.kb1 = kblocks;
     uint32_t c = w / ft_count;
     it.ft = w - c * ft_count;
     uint4 ch = a.chunks[c];
@@ -169,6 +201,7 @@ __device__ __forceinline__ void ws_item(const WsArgs &a, uint32_t w, uint32_t ft
     it.row0 = ch.y;
     it.ntok = ch.z;
     it.nvalid = ch.w;
+    return true;
 }
 
 template <int MODE, int PAIR>
@@ -185,8 +218,8 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     volatile uint32_t *abort = &bars->abort;
 
     // feature tiles: SwiGLU 64 outputs (64 gate + 64 up rows) per CTA, otherwise 128 weight rows per CTA
-    const uint32_t ft_count = MODE == MOE_MM_SWIGLU_F16 ? (a.n / 2u) / (64u * PAIR) : a.n / (128u * PAIR);
-    const uint32_t total = *a.n_chunks * ft_count;
+    const uint32_t ft_count = MODE == MOE_MM_SWIGLU_F16 ? (a.n / 2u) / (64u * PAIR) : (a.n + 128u * PAIR - 1u) / (128u * PAIR);
+    const uint32_t total = MODE == MM_DENSE ? (a.rows + a.per - 1u) / a.per * ft_count * a.splits : *a.n_chunks * ft_count;
     const uint32_t kblocks = (a.k + BK - 1) / BK;
     const uint32_t cluster_id = blockIdx.x / PAIR, n_clusters = gridDim.x / PAIR;
 
@@ -236,12 +269,12 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             bool ok = true;
             for (uint32_t w = cluster_id; w < total && ok; w += n_clusters) {
                 WsItem it;
-                ws_item(a, w, ft_count, it);
+                if (!ws_item<MODE>(a, w, ft_count, kblocks, it)) continue;
                 const uint32_t half = it.ntok / PAIR;            // token rows this CTA loads
                 const uint32_t xbytes = x_rows_loaded(half) * (BK * 2u);
                 const int32_t f0 = (int32_t)((it.ft * PAIR + rank) * (MODE == MOE_MM_SWIGLU_F16 ? 64u : 128u));
                 const int32_t xrow = (int32_t)(it.row0 + rank * half);
-                for (uint32_t kb = 0; kb < kblocks; kb += 1, gstep += 1) {
+                for (uint32_t kb = it.kb0; kb < it.kb1; kb += 1, gstep += 1) {
                     if (gstep % NPROD != turn_of) continue;
                     s = gstep % G::STAGES;
                     ph = (gstep / G::STAGES) & 1u;
@@ -287,13 +320,13 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             bool ok = true;
             for (uint32_t w = cluster_id; w < total && ok; w += n_clusters) {
                 WsItem it;
-                ws_item(a, w, ft_count, it);
+                if (!ws_item<MODE>(a, w, ft_count, kblocks, it)) continue;
                 const uint32_t as = n_item & 1u, aph = (n_item >> 1) & 1u;
                 if (!mbar_wait(smem_u32(&bars->tmem_empty[as]), aph ^ 1u, abort, a.status, 12, a.wait_ns)) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + as * MAX_TOK;
                 const uint32_t idesc = umma_idesc(128u * PAIR, it.ntok);
-                for (uint32_t kb = 0; kb < kblocks; kb += 1, gstep += 1) {
+                for (uint32_t kb = it.kb0; kb < it.kb1; kb += 1, gstep += 1) {
                     const uint32_t s = gstep % G::STAGES;
                     if (((ready >> s) & 1u) == 0 &&
                         !mbar_ring_wait<G::STAGES>(bars->full, gstep, ready, abort, a.status, 13, a.wait_ns)) {
@@ -307,8 +340,8 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     if (elect_one()) {
 #pragma unroll
                         for (uint32_t kk = 0; kk < BK / 16; kk += 1) {
-                            if (PAIR == 2) umma_f16_pair(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-                            else umma_f16(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                            if (PAIR == 2) umma_f16_pair(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, ((kb - it.kb0) | kk) != 0 ? 1u : 0u);
+                            else umma_f16(tmem_d, ad + 2ull * kk, bd + 2ull * kk, idesc, ((kb - it.kb0) | kk) != 0 ? 1u : 0u);
                         }
                         if (PAIR == 2) umma_commit_both(smem_u32(&bars->empty[s]));  // frees the stage in both CTAs
                         else umma_commit(smem_u32(&bars->empty[s]));
@@ -330,9 +363,11 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const uint32_t ew = warp - 2u;   // 0..3: which rows of the turn-round tile this warp stores
         const uint32_t empty_leader = PAIR == 2 ? map_to_cta(smem_u32(&bars->tmem_empty[0]), 0) : smem_u32(&bars->tmem_empty[0]);
         uint32_t n_item = 0, tb = 0;
+        float scale = 1.0f;  // a power of two: partial sums scaled one by one add up to the scaled sum
+        if (MODE == MM_DENSE) scale = 1.0f / (moe_slot_scale(a.amax, a.sa) * moe_slot_scale(a.amax, a.sb));
         for (uint32_t w = cluster_id; w < total; w += n_clusters) {
             WsItem it;
-            ws_item(a, w, ft_count, it);
+            if (!ws_item<MODE>(a, w, ft_count, kblocks, it)) continue;
             const uint32_t as = n_item & 1u, aph = (n_item >> 1) & 1u;
             bool ok = true;
             if (lane == 0) ok = mbar_wait(smem_u32(&bars->tmem_full[as]), aph, abort, a.status, 14, a.wait_ns);
@@ -374,42 +409,63 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     tb ^= 1u;
                 }
             } else if (MODE == MOE_MM_F16) {
-                const uint32_t fl = q * 32u + lane;
-                __half *out = reinterpret_cast<__half *>(a.C) + (size_t)it.row0 * a.ldc + (it.ft * PAIR + rank) * 128u + (lane & 15u) * 8u;
+                // Each warp turns its own 32 features x 32 tokens round: fragments as the tensor core's 16x256b loads
+                // give them (a lane: two neighbouring tokens of features lane/4 and lane/4 + 8), packed to fp16, go
+                // through stmatrix.trans, so that a token's 32 features lie in a row of shared memory; no barrier
+                // with the other warps.  With the relaxed arrival below, 16384 x 2048 outputs of top-10 of 512 experts, K 512:
+                // 526 us with 2-byte stores into a tile of all four warps, 429 us this way; K 768, 4096 x top-8: 126, 115.
+                uint8_t *tp = turn + ew * (ET * PITCH_T);
+                const uint32_t st_addr = smem_u32(tp) + (lane & 7u) * PITCH_T + (lane >> 3) * 16u;
+                const uint8_t *ld = tp + (lane >> 2) * PITCH_T + (lane & 3u) * 16u;
+                __half *out = reinterpret_cast<__half *>(a.C) + (size_t)(it.row0 + (lane >> 2)) * a.ldc +
+                              (it.ft * PAIR + rank) * 128u + q * 32u + (lane & 3u) * 8u;
 #pragma unroll 1
                 for (uint32_t cch = 0; cch < nch; cch += 1) {
-                    uint32_t v[32];
-                    tmem_ld32(taddr + cch * ET, v);
+                    uint32_t lo[16], hi[16];  // features 0..15 and 16..31 of this warp
+                    tmem_ld_16x256b_x4(taddr + cch * ET, lo);
+                    tmem_ld_16x256b_x4(taddr + (16u << 16) + cch * ET, hi);
                     tmem_ld_wait();
-                    uint8_t *tp = turn + tb * ET * PITCH_F16;
-                    __half *mine = reinterpret_cast<__half *>(tp) + fl;
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; j += 1) mine[j * (PITCH_F16 / 2u)] = __float2half_rn(__uint_as_float(v[j]));
-                    epi_sync();
-                    const uint32_t t0c = cch * ET;
+                    __syncwarp();  // the previous chunk has been read
 #pragma unroll
                     for (uint32_t i = 0; i < 4; i += 1) {
-                        const uint32_t r = ew * 8u + i * 2u + (lane >> 4);
-                        if (t0c + r < it.nvalid) {
-                            const uint4 val = *reinterpret_cast<const uint4 *>(tp + r * PITCH_F16 + (lane & 15u) * 16u);
-                            *reinterpret_cast<uint4 *>(out + (size_t)(t0c + r) * a.ldc) = val;
-                        }
+                        stmatrix_x4_trans(st_addr + i * 8u * PITCH_T,
+                                          pack_h2(__uint_as_float(lo[4 * i]), __uint_as_float(lo[4 * i + 1])),
+                                          pack_h2(__uint_as_float(lo[4 * i + 2]), __uint_as_float(lo[4 * i + 3])),
+                                          pack_h2(__uint_as_float(hi[4 * i]), __uint_as_float(hi[4 * i + 1])),
+                                          pack_h2(__uint_as_float(hi[4 * i + 2]), __uint_as_float(hi[4 * i + 3])));
                     }
-                    tb ^= 1u;
+                    __syncwarp();
+                    const uint32_t t0 = cch * ET + (lane >> 2);
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; i += 1) {
+                        const uint4 val = *reinterpret_cast<const uint4 *>(ld + i * 8u * PITCH_T);
+                        if (t0 + i * 8u < it.nvalid) *reinterpret_cast<uint4 *>(out + (size_t)(cch * ET + i * 8u) * a.ldc) = val;
+                    }
                 }
             } else {
                 // fp32 output: 32 lanes = 32 neighbouring features = one 128-byte piece of a token's row per store
                 const uint32_t cfeat = (it.ft * PAIR + rank) * 128u + q * 32u + lane;
+                // dense form: the last pair may reach beyond n (n is a multiple of 128, not of 256)
+                const uint32_t nvalid = MODE == MM_DENSE && cfeat >= a.n ? 0u : it.nvalid;
+                float *C = reinterpret_cast<float *>(a.C) + (MODE == MM_DENSE ? (size_t)it.split * a.rows * a.ldc : 0u);
 #pragma unroll 1
                 for (uint32_t cch = 0; cch < nch; cch += 1) {
                     uint32_t v[32];
                     tmem_ld32(taddr + cch * ET, v);
                     tmem_ld_wait();
                     const uint32_t t0c = cch * ET;
-                    float *out = reinterpret_cast<float *>(a.C) + (size_t)(it.row0 + t0c) * a.ldc + cfeat;
+                    float *out = C + (size_t)(it.row0 + t0c) * a.ldc + cfeat;
+                    if (t0c + 32u <= nvalid) {  // one test for the whole chunk: a test per store costs ten times the stores
 #pragma unroll
-                    for (uint32_t j = 0; j < 32; j += 1) {
-                        if (t0c + j < it.nvalid) out[(size_t)j * a.ldc] = __uint_as_float(v[j]);
+                        for (uint32_t j = 0; j < 32; j += 1) {
+                            *out = MODE == MM_DENSE ? __uint_as_float(v[j]) * scale : __uint_as_float(v[j]);
+                            out += a.ldc;
+                        }
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j += 1) {
+                            if (t0c + j < nvalid) out[(size_t)j * a.ldc] = MODE == MM_DENSE ? __uint_as_float(v[j]) * scale : __uint_as_float(v[j]);
+                        }
                     }
                 }
             }
@@ -439,6 +495,22 @@ __global__ void __launch_bounds__(512)
 moe_chunk_kernel(const uint32_t *__restrict__ count, const uint32_t *__restrict__ off, uint32_t experts,
                  uint4 *__restrict__ chunks, uint32_t *__restrict__ n_chunks, uint32_t max_chunks) {
     moe_chunk_body(count, off, experts, chunks, n_chunks, max_chunks);
+}
+
+// C = the sum of the partial products of a split K, in split order.  n and with it every row is a multiple of four.
+__global__ void __launch_bounds__(256)
+moe_ksum_kernel(const float4 *__restrict__ part, float4 *__restrict__ C, uint32_t total4, uint32_t splits) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= total4) return;
+    float4 acc = __ldcg(part + i);
+    for (uint32_t p = 1; p < splits; p += 1) {
+        const float4 v = __ldcg(part + (size_t)p * total4 + i);
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+    }
+    C[i] = acc;
 }
 
 template <int MODE, int PAIR>
@@ -491,7 +563,7 @@ void moe_launch_mm_ws(moe_cuda_ctx *c, int mode, int pair, const void *X, uint32
                                   : !moe_tmap_2d_f16(c, &tmW, W, (uint64_t)experts_in_W * n, k, 128)) return;
     moe_xmaps tmX;
     if (!moe_tmap_tokens_f16(c, &tmX, X, rows_x, k)) return;
-    WsArgs a;
+    WsArgs a = {};
     a.C = C;
     a.chunks = (const uint4 *)chunks;
     a.n_chunks = n_chunks;
@@ -516,4 +588,80 @@ void moe_launch_mm_ws(moe_cuda_ctx *c, int mode, int pair, const void *X, uint32
     WS_CASE(MOE_MM_F32, 1)
     WS_CASE(MOE_MM_F32, 2)
 #undef WS_CASE
+}
+
+namespace {
+// Rows per item and K splits of the dense form: the pair with the least estimated time.  Unit: 128 bytes loaded into
+// an SM (1.8 ns at the 70 B/ns that an SM gets from L2).  A K step brings 128 weight rows and half of the item's token
+// rows of 128 bytes; an epilogue stores 512 bytes per token and is hidden but for the last one; a split costs a second
+// launch (4 us) and its partial sums a write and a read through L2 (5 TB/s).
+// 3001 x 384, K 8192: 34 us as 3 splits against 64 us whole on the token-major kernel; 384 x 384: 16 against 64 us.
+void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t kblocks, uint32_t clusters, bool tiled) {
+    const uint32_t nch0 = (rows + MAX_TOK - 1u) / MAX_TOK;
+    uint64_t best = ~0ull;
+    for (uint32_t i = 0; i < (tiled ? 3u : 4u); i += 1) {
+        // tile schedule given: parts of its 128-row tiles; else the fewest chunks, and finer cuts where these are few
+        const uint32_t nch = nch0 * (i + 1u);
+        const uint32_t per = tiled ? MOE_TILE >> i : ((rows + nch - 1u) / nch + 15u) & ~15u;
+        const uint64_t items = (uint64_t)((rows + per - 1u) / per) * ft;
+        for (uint32_t s = 1; s <= (tiled ? 1u : 32u) && (s == 1 || s * 4u <= kblocks); s += 1) {
+            const uint32_t ks = (kblocks + s - 1u) / s;
+            const uint64_t waves = (items * s + clusters - 1u) / clusters;
+            uint64_t t = waves * ks * (128u + per / 2u) + per * 4u;
+            if (s > 1) t += 2200u + (uint64_t)s * rows * n * 8u / 9000u;
+            if (t < best) {
+                best = t;
+                a.per = per;
+                a.ksplit = ks;
+                a.splits = (kblocks + ks - 1u) / ks;  // no empty split
+            }
+            if (items * s >= 4u * (uint64_t)clusters) break;  // the last wave no longer matters
+        }
+    }
+}
+}  // namespace
+
+// Dense product on the same kernel, pairs of CTAs only: C[rows x n] = X[rows x k] * W[e][n x k]^T / scales, where e is 0
+// or, with `tiles`, the expert of the 128-row tile.
+//   tiles == NULL: chunks of up to 256 rows; K may be split, the fp32 partial sums are then added in split order by a
+//     second kernel.
+//   tiles != NULL: chunks of 128, 64 or 32 rows, K whole, no scratch.
+void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C, const uint32_t *amax, const uint32_t *tiles,
+                         uint32_t rows, uint32_t n, uint32_t k, uint32_t sa, uint32_t sb, uint32_t experts_in_W) {
+    if (!MOE_LIVE(c)) return;
+    MOE_REQUIRE(c, X != NULL && W != NULL && C != NULL, "mm_dense: null buffer");
+    MOE_REQUIRE(c, rows >= 1 && n % 128u == 0 && n >= 128u && k % 8u == 0 && k >= 8u, "mm_dense: rows %u n %u k %u", rows, n, k);
+    MOE_REQUIRE(c, experts_in_W >= 1 && (uint64_t)experts_in_W * n < (1ull << 31) && rows < (1u << 31), "mm_dense: size");
+    MOE_REQUIRE(c, (sa == MDA_PC_NO_SLOT && sb == MDA_PC_NO_SLOT) || amax != NULL, "mm_dense: scale slot without amax");
+    MOE_REQUIRE(c, ((uintptr_t)C & 15) == 0, "mm_dense: C not 16-byte aligned");
+    CUtensorMap tmW;
+    moe_xmaps tmX;
+    if (!moe_tmap_2d_f16(c, &tmW, W, (uint64_t)experts_in_W * n, k, 128) || !moe_tmap_tokens_f16(c, &tmX, X, rows, k)) return;
+    const uint32_t clusters = (uint32_t)c->sm_count / 2u, ft = (n + 255u) / 256u, kblocks = (k + BK - 1u) / BK;
+    WsArgs a = {};
+    ws_dense_plan(a, rows, n, ft, kblocks, clusters, tiles != NULL);
+    a.C = C;
+    if (a.splits > 1) {
+        a.C = moe_scratch(c, MOE_SCR_STAGE, (size_t)a.splits * rows * n * 4);
+        if (a.C == NULL) return;
+    }
+    a.n = n;
+    a.k = k;
+    a.ldc = n;
+    a.rows = rows;
+    a.tiles = tiles;
+    a.experts = experts_in_W;
+    a.amax = amax;
+    a.sa = sa;
+    a.sb = sb;
+    a.status = c->dev_status_dev;
+    a.wait_ns = c->wait_ns;
+    const uint64_t total = (uint64_t)((rows + a.per - 1u) / a.per) * ft * a.splits;
+    MOE_REQUIRE(c, total < (1ull << 31), "mm_dense: too many tiles");
+    ws_launch<MM_DENSE, 2>(c, tmW, tmX, a, (uint32_t)(total < clusters ? total : clusters) * 2u);
+    if (a.splits > 1 && MOE_LIVE(c)) {
+        const uint32_t total4 = rows * (n / 4u);
+        moe_ksum_kernel<<<(total4 + 255u) / 256u, 256, 0, c->stream>>>((const float4 *)a.C, (float4 *)C, total4, a.splits);
+        MOE_LAUNCHED(c);
+    }
 }

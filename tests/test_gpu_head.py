@@ -69,7 +69,11 @@ def test_elem_op1(ctx, oracle):
     assert np.all(np.abs(got - ref) <= 1e-6 * np.abs(ref) + 1e-7)
 
 
-@pytest.mark.parametrize("rows,n,k,slot", [(200, 384, 1024, True), (64, 128, 320, False), (256, 1280, 256, True), (1, 128, 8, False)])
+@pytest.mark.parametrize("rows,n,k,slot", [(200, 384, 1024, True), (64, 128, 320, False), (256, 1280, 256, True), (1, 128, 8, False),
+                                           # K split (evenly, with a short last part), a last pair of feature tiles with one tile
+                                           # in it, chunks of several sizes with a ragged last one, more items than clusters
+                                           (384, 384, 8192, True), (3, 128, 4104, False), (257, 384, 520, True), (1003, 384, 2048, False),
+                                           (513, 256, 320, True), (700, 19328, 72, False)])
 def test_dense(ctx, oracle, rows, n, k, slot):
     """mda_qwen_mm: any row count (rows beyond A read as zero, rows beyond C are not written)."""
     rng = np.random.default_rng(rows + n)

@@ -152,6 +152,7 @@ def _f16(rng, shape, std):
 @pytest.mark.parametrize("m,n,k,E,sa", [
     (128, 128, 64, 1, False), (128, 256, 64, 1, False), (256, 384, 128, 3, False), (512, 1024, 256, 4, True),
     (384, 640, 96, 2, False), (1280, 256, 2048, 8, False), (256, 2048, 768, 5, True), (128, 128, 8, 1, False),
+    (4736, 256, 128, 3, True), (4864, 256, 128, 3, True), (2048, 384, 200, 1, False),  # either side of the idle-SM rule
 ])
 def test_mm(ctx, oracle, mc, m, n, k, E, sa):
     """moe_cuda_mm against the oracle's product: same tile schedule, skipped tiles untouched,
