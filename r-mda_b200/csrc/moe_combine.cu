@@ -4,24 +4,51 @@
 #include "moe_common.cuh"
 
 #define CB_THREADS 256
-#define CB_MAXV 8  // float4 per thread kept for the fused norm: d <= 8192
+#define CB_KEEP 32  // values per thread kept for the fused norm: d <= 8192
+#define CB_TERMS 8  // expert rows whose loads a thread has in flight together
 
 __device__ __forceinline__ float moe_sigmoid(float v) {  // shader/moe_combine.comp:22-24
     return 1.0f / (1.0f + expf(-v));
 }
 
-__device__ __forceinline__ float4 moe_load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
-__device__ __forceinline__ float4 moe_load4(const __half *p) {
-    uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
-    float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&raw.x));
-    float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&raw.y));
-    return make_float4(a.x, a.y, b.x, b.y);
+// V neighbouring values of a row, 8 to 16 bytes, as fetched and as floats.
+template <typename YT, int V> struct moe_vec;
+template <> struct moe_vec<float, 4> { typedef float4 raw; };
+template <> struct moe_vec<__half, 4> { typedef uint2 raw; };
+template <> struct moe_vec<__half, 8> { typedef uint4 raw; };
+template <typename YT, int V>
+__device__ __forceinline__ typename moe_vec<YT, V>::raw moe_fetch(const YT *p) {
+    return __ldg(reinterpret_cast<const typename moe_vec<YT, V>::raw *>(p));
+}
+__device__ __forceinline__ void moe_floats(float4 r, float (&f)[4]) {
+    f[0] = r.x; f[1] = r.y; f[2] = r.z; f[3] = r.w;
+}
+__device__ __forceinline__ void moe_floats2(uint32_t r, float *f) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r));
+    f[0] = a.x; f[1] = a.y;
+}
+__device__ __forceinline__ void moe_floats(uint2 r, float (&f)[4]) {
+    moe_floats2(r.x, f); moe_floats2(r.y, f + 2);
+}
+__device__ __forceinline__ void moe_floats(uint4 r, float (&f)[8]) {
+    moe_floats2(r.x, f); moe_floats2(r.y, f + 2); moe_floats2(r.z, f + 4); moe_floats2(r.w, f + 6);
+}
+// acc += w * v, multiply and add rounded separately
+template <int V>
+__device__ __forceinline__ void moe_axpy(float (&acc)[V], float w, const float (&v)[V]) {
+#pragma unroll
+    for (int i = 0; i < V; i += 1) acc[i] = __fadd_rn(acc[i], __fmul_rn(w, v[i]));
 }
 
 // One block per row (shader/moe_combine.comp:26-40 uses one thread per element).
 // acc = sum_j wt[r,j] * y[slot[r,j], c] in j order with separately rounded
 // multiply and add, as the expression is written in the shader (:32-34).
-template <typename YT, bool NORM, bool PEER>
+// Bound by HBM for many rows and by the chain of loads for few: a thread takes V values of 16 bytes where the row
+// allows it, and the loads of up to CB_TERMS expert rows are issued before the first is used (one at a time, 16 rows
+// of 2048 with the norm took 11.2 us); the values kept for the norm are indexed statically, so that they stay in
+// registers (2048 rows: 37 us before, 23 us now; 16 rows 4.5 us).
+// NORM: 0, or the fused norm's passes of CB_THREADS * V columns over the row.
+template <typename YT, int NORM, bool PEER, int V>
 __global__ void __launch_bounds__(CB_THREADS)
 moe_combine_kernel(moe_combine_args a) {
     __shared__ uint32_t s_slot[MOE_MAX_TOPK];
@@ -74,49 +101,67 @@ moe_combine_kernel(moe_combine_args a) {
         __syncthreads();
         const uint32_t terms = (PEER && a.per_gpu) ? s_terms : a.topk;
         float sg = s_f[7];
-        float4 keep[NORM ? CB_MAXV : 1];
+        constexpr int ITS = NORM ? NORM : 1;  // unrolled where their values are kept
+        float keep[ITS][V];
         float ss = 0.0f;
-        uint32_t it = 0;
-        for (uint32_t c = threadIdx.x * 4u; c < a.d; c += CB_THREADS * 4u, it += 1) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t j = 0; j < terms; j += 1) {
-                if (s_slot[j] == ~0u) continue;
-                float4 v = moe_load4((PEER ? s_y[j] : y) + (size_t)s_slot[j] * a.d + c);
-                float w = s_wt[j];
-                acc.x = __fadd_rn(acc.x, __fmul_rn(w, v.x));
-                acc.y = __fadd_rn(acc.y, __fmul_rn(w, v.y));
-                acc.z = __fadd_rn(acc.z, __fmul_rn(w, v.z));
-                acc.w = __fadd_rn(acc.w, __fmul_rn(w, v.w));
-            }
-            if (a.sh != NULL) {
-                float4 v = moe_load4(a.sh + (size_t)r * a.d + c);
-                acc.x = __fadd_rn(acc.x, __fmul_rn(sg, v.x));
-                acc.y = __fadd_rn(acc.y, __fmul_rn(sg, v.y));
-                acc.z = __fadd_rn(acc.z, __fmul_rn(sg, v.z));
-                acc.w = __fadd_rn(acc.w, __fmul_rn(sg, v.w));
-            }
-            if (NORM) {
-                float4 xv = moe_load4(a.x16 + (size_t)r * a.d + c);
-                float f = s_f[0];
-                float4 v;
-                v.x = __fadd_rn(xv.x, __fmul_rn(__fmul_rn(acc.x, 2.0f), f));
-                v.y = __fadd_rn(xv.y, __fmul_rn(__fmul_rn(acc.y, 2.0f), f));
-                v.z = __fadd_rn(xv.z, __fmul_rn(__fmul_rn(acc.z, 2.0f), f));
-                v.w = __fadd_rn(xv.w, __fmul_rn(__fmul_rn(acc.w, 2.0f), f));
-                keep[it] = v;
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
-            if (a.h != NULL) {
-                for (uint32_t s = 0; s < a.hc; s += 1) {  // :36-38
-                    float f = a.hc <= 7 ? s_f[s]
-                                        : moe_sigmoid((a.inj != NULL ? a.inj[(size_t)r * a.inj_stride + a.inj_off + s] : 0.0f) / (float)a.hc);
-                    float4 *hp = reinterpret_cast<float4 *>(a.h + ((size_t)r * a.hc + s) * a.d + c);
-                    float4 hv = *hp;
-                    hv.x = __fadd_rn(hv.x, __fmul_rn(__fmul_rn(acc.x, 2.0f), f));
-                    hv.y = __fadd_rn(hv.y, __fmul_rn(__fmul_rn(acc.y, 2.0f), f));
-                    hv.z = __fadd_rn(hv.z, __fmul_rn(__fmul_rn(acc.z, 2.0f), f));
-                    hv.w = __fadd_rn(hv.w, __fmul_rn(__fmul_rn(acc.w, 2.0f), f));
-                    *hp = hv;
+        for (uint32_t c0 = 0; c0 < a.d; c0 += CB_THREADS * V * ITS) {
+#pragma unroll
+            for (int it = 0; it < ITS; it += 1) {
+                const uint32_t c = c0 + (it * CB_THREADS + threadIdx.x) * V;
+                if (c >= a.d) break;
+                float acc[V], f[V];
+#pragma unroll
+                for (int i = 0; i < V; i += 1) acc[i] = 0.0f;
+                for (uint32_t j0 = 0; j0 < terms; j0 += CB_TERMS) {
+                    typename moe_vec<YT, V>::raw v[CB_TERMS];
+#pragma unroll
+                    for (uint32_t j = 0; j < CB_TERMS; j += 1) {
+                        if (j0 + j < terms && s_slot[j0 + j] != ~0u)
+                            v[j] = moe_fetch<YT, V>((PEER ? s_y[j0 + j] : y) + (size_t)s_slot[j0 + j] * a.d + c);
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < CB_TERMS; j += 1) {
+                        if (j0 + j >= terms || s_slot[j0 + j] == ~0u) continue;
+                        moe_floats(v[j], f);
+                        moe_axpy<V>(acc, s_wt[j0 + j], f);
+                    }
+                }
+                if (a.sh != NULL) {
+#pragma unroll
+                    for (int i = 0; i < V; i += 4) {
+                        const float4 v = __ldg(reinterpret_cast<const float4 *>(a.sh + (size_t)r * a.d + c + i));
+                        acc[i] = __fadd_rn(acc[i], __fmul_rn(sg, v.x));
+                        acc[i + 1] = __fadd_rn(acc[i + 1], __fmul_rn(sg, v.y));
+                        acc[i + 2] = __fadd_rn(acc[i + 2], __fmul_rn(sg, v.z));
+                        acc[i + 3] = __fadd_rn(acc[i + 3], __fmul_rn(sg, v.w));
+                    }
+                }
+                if (NORM) {
+                    moe_floats(moe_fetch<__half, V>(a.x16 + (size_t)r * a.d + c), f);
+#pragma unroll
+                    for (int i = 0; i < V; i += 1) {
+                        keep[it][i] = __fadd_rn(f[i], __fmul_rn(__fmul_rn(acc[i], 2.0f), s_f[0]));
+                        ss += keep[it][i] * keep[it][i];
+                    }
+                }
+                if (a.h != NULL) {
+#pragma unroll 2
+                    for (uint32_t s = 0; s < a.hc; s += 1) {  // :36-38
+                        const float g = a.hc <= 7 ? s_f[s]
+                                                  : moe_sigmoid((a.inj != NULL ? a.inj[(size_t)r * a.inj_stride + a.inj_off + s] : 0.0f) / (float)a.hc);
+                        float4 *hp = reinterpret_cast<float4 *>(a.h + ((size_t)r * a.hc + s) * a.d + c);
+                        float4 hv[V / 4];
+#pragma unroll
+                        for (int i = 0; i < V / 4; i += 1) hv[i] = hp[i];
+#pragma unroll
+                        for (int i = 0; i < V / 4; i += 1) {
+                            hv[i].x = __fadd_rn(hv[i].x, __fmul_rn(__fmul_rn(acc[4 * i], 2.0f), g));
+                            hv[i].y = __fadd_rn(hv[i].y, __fmul_rn(__fmul_rn(acc[4 * i + 1], 2.0f), g));
+                            hv[i].z = __fadd_rn(hv[i].z, __fmul_rn(__fmul_rn(acc[4 * i + 2], 2.0f), g));
+                            hv[i].w = __fadd_rn(hv[i].w, __fmul_rn(__fmul_rn(acc[4 * i + 3], 2.0f), g));
+                            hp[i] = hv[i];
+                        }
+                    }
                 }
             }
         }
@@ -130,15 +175,15 @@ moe_combine_kernel(moe_combine_args a) {
 #pragma unroll
             for (uint32_t w = 0; w < CB_THREADS / 32; w += 1) tot += s_red[w];
             float inv = 1.0f / sqrtf(tot / (float)a.d + a.eps);
-            it = 0;
-            for (uint32_t c = threadIdx.x * 4u; c < a.d; c += CB_THREADS * 4u, it += 1) {
-                float4 v = keep[it];
-                __half2 lo = __floats2half2_rn(v.x * inv, v.y * inv);
-                __half2 hi = __floats2half2_rn(v.z * inv, v.w * inv);
-                uint2 out;
-                out.x = *reinterpret_cast<uint32_t *>(&lo);
-                out.y = *reinterpret_cast<uint32_t *>(&hi);
-                *reinterpret_cast<uint2 *>(a.y16 + (size_t)r * a.d + c) = out;
+#pragma unroll
+            for (int it = 0; it < ITS; it += 1) {
+                const uint32_t c = (it * CB_THREADS + threadIdx.x) * V;
+                if (c >= a.d) break;
+                __align__(16) __half2 o[V / 2];
+#pragma unroll
+                for (int i = 0; i < V / 2; i += 1) o[i] = __floats2half2_rn(keep[it][2 * i] * inv, keep[it][2 * i + 1] * inv);
+                *reinterpret_cast<typename moe_vec<__half, V>::raw *>(a.y16 + (size_t)r * a.d + c) =
+                    *reinterpret_cast<const typename moe_vec<__half, V>::raw *>(o);
             }
         }
         __syncthreads();  // the row's tables are rewritten by the next pass
@@ -149,9 +194,9 @@ moe_combine_kernel(moe_combine_args a) {
 // kernel can only join an SM whose shared-memory carve-out matches its own, and the products run
 // with the maximum carve-out.
 void moe_overlap_prepare_combine(moe_cuda_ctx *c) {
-    MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_combine_kernel<__half, false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_combine_kernel<__half, 0, true, 8>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
-    MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_combine_kernel<__half, true, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_combine_kernel<__half, CB_KEEP / 8, true, 8>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
 }
 
@@ -169,7 +214,7 @@ void moe_launch_combine(moe_cuda_ctx *c, const moe_combine_args &a) {
     MOE_REQUIRE(c, ((uintptr_t)a.y & 15) == 0 && ((uintptr_t)a.h & 15) == 0 && ((uintptr_t)a.sh & 15) == 0,
                 "combine: buffers not 16-byte aligned");
     if (a.y16 != NULL) {
-        MOE_REQUIRE(c, a.x16 != NULL && a.hc == 1 && a.d <= CB_THREADS * 4 * CB_MAXV, "combine: fused norm needs x16, hc 1, d <= 8192");
+        MOE_REQUIRE(c, a.x16 != NULL && a.hc == 1 && a.d <= CB_THREADS * CB_KEEP, "combine: fused norm needs x16, hc 1, d <= 8192");
     }
     if (a.rows == 0) return;
     const bool peer = a.y_peers != NULL;
@@ -178,15 +223,24 @@ void moe_launch_combine(moe_cuda_ctx *c, const moe_combine_args &a) {
     // leave room for another token slice's product CTAs, measured 115 us against 47 us for the return over 2 GPUs
     // and 0.686 ms against 0.670 ms per layer over 8.)
     const uint32_t grid = a.rows;
+    // 16 bytes of fp16 at a time; rows of 4 values more than a multiple of 8, or a caller's buffer on 8 bytes, take 8 bytes
+    const bool wide = a.y_is_f16 && a.d % 8u == 0 && (((uintptr_t)a.x16 | (uintptr_t)a.y16) & 15) == 0;
+#define CB_RUN(YT, NORM, PEER, V) moe_combine_kernel<YT, NORM, PEER, V><<<grid, CB_THREADS, 0, c->stream>>>(a)
     if (a.y16 != NULL) {
-        if (peer) moe_combine_kernel<__half, true, true><<<grid, CB_THREADS, 0, c->stream>>>(a);
-        else if (a.y_is_f16) moe_combine_kernel<__half, true, false><<<grid, CB_THREADS, 0, c->stream>>>(a);
-        else moe_combine_kernel<float, true, false><<<grid, CB_THREADS, 0, c->stream>>>(a);
+        if (peer && wide) CB_RUN(__half, CB_KEEP / 8, true, 8);
+        else if (peer) CB_RUN(__half, CB_KEEP / 4, true, 4);
+        else if (wide && a.d <= CB_THREADS * 8) CB_RUN(__half, 1, false, 8);  // a third fewer registers: more rows in flight
+        else if (wide) CB_RUN(__half, CB_KEEP / 8, false, 8);
+        else if (a.y_is_f16) CB_RUN(__half, CB_KEEP / 4, false, 4);
+        else CB_RUN(float, CB_KEEP / 4, false, 4);
     } else {
-        if (peer) moe_combine_kernel<__half, false, true><<<grid, CB_THREADS, 0, c->stream>>>(a);
-        else if (a.y_is_f16) moe_combine_kernel<__half, false, false><<<grid, CB_THREADS, 0, c->stream>>>(a);
-        else moe_combine_kernel<float, false, false><<<grid, CB_THREADS, 0, c->stream>>>(a);
+        if (peer && wide) CB_RUN(__half, 0, true, 8);
+        else if (peer) CB_RUN(__half, 0, true, 4);
+        else if (wide) CB_RUN(__half, 0, false, 8);
+        else if (a.y_is_f16) CB_RUN(__half, 0, false, 4);
+        else CB_RUN(float, 0, false, 4);
     }
+#undef CB_RUN
     MOE_LAUNCHED(c);
 }
 

@@ -178,3 +178,26 @@ def test_many_tensor_maps_in_one_context(ctx, mc, synth, oracle):
     check(run_layer(ctx, mc, small, part), oracle.layer(part.proj, part.x16, part.wgu, part.wdown, cfg.K))
     again = run_layer(ctx, mc, cfg, inp)
     assert np.array_equal(again["h"], first["h"])
+
+
+@pytest.mark.parametrize("d,K,shift", [(128, 2, 0), (256, 10, 4), (2048, 8, 0), (2048, 9, 4), (2176, 16, 0), (8192, 3, 0), (8192, 3, 4)])
+def test_fused_norm_widths(ctx, mc, oracle, d, K, shift):
+    """Fused residual + RMSNorm over rows of one and several passes, more expert rows than are loaded together, and an
+    output buffer `shift` fp16 values off 16 bytes, against the same layer's fp32 residual output normalised here."""
+    rng = np.random.default_rng(d + K)
+    T, E, I = 19, 16, 128
+    f16 = lambda *s, std: ctx.upload((rng.standard_normal(s) * std).astype(np.float16).view(np.uint16))
+    x = rng.standard_normal((T, d)).astype(np.float16)
+    a = dict(rows=T, d=d, experts=E, topk=K, inter=I, shared=0, pstride=E + 4, hc=1,
+             proj=ctx.upload(rng.standard_normal((T, E + 4)).astype(np.float32)), x16=ctx.upload(x.view(np.uint16)),
+             wgu=f16(E, 2 * I, d, std=0.05), wdown=f16(E, d, I, std=0.3))
+    d_h, d_y = ctx.zeros(T * d * 4), ctx.upload(np.full(T * d + 8, 0x7bff, np.uint16))
+    ctx.layer(h=d_h, **a)
+    ctx.layer(y16=d_y.ptr + 2 * shift, eps=1e-6, **a)
+    ctx.flush()
+    v = x.astype(np.float32) + d_h.read(np.float32, (T, d))
+    ref = v / np.sqrt((v.astype(np.float64) ** 2).mean(1, keepdims=True) + 1e-6)
+    raw = d_y.read(np.uint16, (T * d + 8,))
+    got = raw[shift:shift + T * d].view(np.float16).reshape(T, d).astype(np.float64)
+    assert np.all(np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) * 1.01 + 2.0 ** -25)   # one rounding to fp16
+    assert np.all(raw[:shift] == 0x7bff) and np.all(raw[shift + T * d:] == 0x7bff)
