@@ -226,23 +226,26 @@ __device__ __forceinline__ void moe_scan_body(const uint32_t *count, uint32_t *o
 #define MOE_CHUNK_TOK 256u
 __device__ __forceinline__ void moe_chunk_body(const uint32_t *count, const uint32_t *off, uint32_t experts, uint4 *chunks,
                                                uint32_t *n_chunks, uint32_t max_chunks) {
-    __shared__ uint32_t csum[512];
-    const uint32_t e = threadIdx.x;
-    uint32_t cnt = 0, nch = 0;
-    if (e < 512u) {
-        cnt = e < experts ? __ldcg(count + e) : 0u;
-        nch = (cnt + MOE_CHUNK_TOK - 1u) / MOE_CHUNK_TOK;
-        csum[e] = nch;
+    __shared__ uint32_t wchunks[16];
+    const uint32_t e = threadIdx.x, lane = e & 31u, warp = e >> 5;
+    const uint32_t cnt = e < experts && e < 512u ? __ldcg(count + e) : 0u;
+    const uint32_t nch = (cnt + MOE_CHUNK_TOK - 1u) / MOE_CHUNK_TOK;
+    uint32_t incl = nch;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
+    if (lane == 31 && warp < 16) wchunks[warp] = incl;
     __syncthreads();
-    for (uint32_t o = 1; o < 512; o <<= 1) {
-        uint32_t v = (e < 512u && e >= o) ? csum[e - o] : 0u;
-        __syncthreads();
-        if (e < 512u) csum[e] += v;
-        __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 16; w += 1) {
+        before += w < warp ? wchunks[w] : 0u;
+        all += wchunks[w];
     }
     if (e < 512u && nch != 0) {
-        const uint32_t first = csum[e] - nch;
+        const uint32_t first = before + incl - nch;
         const uint32_t per = ((cnt + nch - 1u) / nch + 15u) & ~15u;
         const uint32_t row0 = __ldcg(off + e);
         for (uint32_t j = 0; j < nch; j += 1) {
@@ -251,7 +254,7 @@ __device__ __forceinline__ void moe_chunk_body(const uint32_t *count, const uint
             if (first + j < max_chunks) chunks[first + j] = make_uint4(e, row0 + start, (valid + 15u) & ~15u, valid);
         }
     }
-    if (e == 511u) *n_chunks = min(csum[511], max_chunks);
+    if (e == 0u) *n_chunks = min(all, max_chunks);
 }
 
 __device__ __forceinline__ float moe_slot_scale(const uint32_t *amax, uint32_t s) {
