@@ -51,6 +51,7 @@ __device__ __forceinline__ void moe_axpy(float (&acc)[V], float w, const float (
 template <typename YT, int NORM, bool PEER, int V>
 __global__ void __launch_bounds__(CB_THREADS)
 moe_combine_kernel(moe_combine_args a) {
+    moe_pdl_begin();
     __shared__ uint32_t s_slot[MOE_MAX_TOPK];
     __shared__ float s_wt[MOE_MAX_TOPK];
     __shared__ float s_f[8];
@@ -225,7 +226,7 @@ void moe_launch_combine(moe_cuda_ctx *c, const moe_combine_args &a) {
     const uint32_t grid = a.rows;
     // 16 bytes of fp16 at a time; rows of 4 values more than a multiple of 8, or a caller's buffer on 8 bytes, take 8 bytes
     const bool wide = a.y_is_f16 && a.d % 8u == 0 && (((uintptr_t)a.x16 | (uintptr_t)a.y16) & 15) == 0;
-#define CB_RUN(YT, NORM, PEER, V) moe_combine_kernel<YT, NORM, PEER, V><<<grid, CB_THREADS, 0, c->stream>>>(a)
+#define CB_RUN(YT, NORM, PEER, V) moe_run(c, moe_combine_kernel<YT, NORM, PEER, V>, grid, CB_THREADS, 0, a)
     if (a.y16 != NULL) {
         if (peer && wide) CB_RUN(__half, CB_KEEP / 8, true, 8);
         else if (peer) CB_RUN(__half, CB_KEEP / 4, true, 4);
@@ -285,6 +286,7 @@ __device__ __forceinline__ float moe_elem(float g, float u, uint32_t op, float s
 // General form: any n, stride, offset and alignment.
 __global__ void moe_swiglu_kernel(const float *__restrict__ a, float *__restrict__ y, uint32_t rows, uint32_t n,
                                   uint32_t astride, uint32_t ao, uint32_t bo, uint32_t op, float scale) {
+    moe_pdl_begin();
     size_t total = (size_t)rows * n;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -299,6 +301,7 @@ template <uint32_t OP>
 __global__ void __launch_bounds__(EL_THREADS)
 moe_swiglu4_kernel(const float4 *__restrict__ a, float4 *__restrict__ y, uint32_t total4, uint32_t n4, uint32_t astride4,
                    uint32_t ao4, uint32_t bo4, float scale) {
+    moe_pdl_begin();
     constexpr uint32_t U = 2;  // two operands: four loads in flight
     const uint32_t i0 = blockIdx.x * (EL_THREADS * U) + threadIdx.x;
     float4 g[U], u[U];
@@ -331,23 +334,24 @@ extern "C" void moe_cuda_swiglu(moe_cuda_ctx_t *c, const float *a, float *y, str
         total / 4 < (1ull << 31)) {
         const uint32_t total4 = (uint32_t)(total / 4), blocks = (total4 + 2u * EL_THREADS - 1u) / (2u * EL_THREADS);
         if (pc.op == 0u)
-            moe_swiglu4_kernel<0><<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)a, (float4 *)y, total4, pc.n / 4u,
+            moe_run(c, moe_swiglu4_kernel<0>, blocks, EL_THREADS, 0, (const float4 *)a, (float4 *)y, total4, pc.n / 4u,
                                                                        pc.astride / 4u, pc.ao / 4u, pc.bo / 4u, pc.scale);
         else
-            moe_swiglu4_kernel<1><<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)a, (float4 *)y, total4, pc.n / 4u,
+            moe_run(c, moe_swiglu4_kernel<1>, blocks, EL_THREADS, 0, (const float4 *)a, (float4 *)y, total4, pc.n / 4u,
                                                                        pc.astride / 4u, pc.ao / 4u, 0, pc.scale);
         MOE_LAUNCHED(c);
         return;
     }
     size_t blocks = (total + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
-    moe_swiglu_kernel<<<(unsigned)blocks, 256, 0, c->stream>>>(a, y, pc.rows, pc.n, pc.astride, pc.ao, pc.bo, pc.op, pc.scale);
+    moe_run(c, moe_swiglu_kernel, (unsigned)blocks, 256, 0, a, y, pc.rows, pc.n, pc.astride, pc.ao, pc.bo, pc.op, pc.scale);
     MOE_LAUNCHED(c);
 }
 
 // n4 float4 from the first 16-byte boundary of x on; the few values before and behind them go to the first threads.
 __global__ void __launch_bounds__(EL_THREADS)
 moe_absmax_kernel(const float *__restrict__ x, uint32_t *__restrict__ amax, uint32_t n, uint32_t head, uint32_t slot) {
+    moe_pdl_begin();
     __shared__ float red[EL_THREADS / 32];
     const uint32_t n4 = (n - head) / 4u, stride = gridDim.x * EL_THREADS;
     const float4 *x4 = reinterpret_cast<const float4 *>(x + head);
@@ -385,7 +389,7 @@ extern "C" void moe_cuda_absmax(moe_cuda_ctx_t *c, const float *x, uint32_t *ama
     if (head > pc.n) head = pc.n;
     uint32_t blocks = (uint32_t)(((uint64_t)pc.n + 4u * EL_VECS * EL_THREADS - 1u) / (4u * EL_VECS * EL_THREADS));
     if (blocks > (uint32_t)c->sm_count * 8u) blocks = (uint32_t)c->sm_count * 8u;
-    moe_absmax_kernel<<<blocks, EL_THREADS, 0, c->stream>>>(x, amax, pc.n, head, pc.slot);
+    moe_run(c, moe_absmax_kernel, blocks, EL_THREADS, 0, x, amax, pc.n, head, pc.slot);
     MOE_LAUNCHED(c);
 }
 
@@ -397,6 +401,7 @@ __device__ __forceinline__ uint2 moe_pack4(float4 v, float s) {
 // General form: any alignment.
 __global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__restrict__ dst, size_t n,
                                     const uint32_t *__restrict__ amax, uint32_t slot) {
+    moe_pdl_begin();
     float s = moe_slot_scale(amax, slot);
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -408,6 +413,7 @@ __global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__res
 __global__ void __launch_bounds__(EL_THREADS)
 moe_cast4_f16_kernel(const float4 *__restrict__ src, uint2 *__restrict__ dst, uint32_t n, const uint32_t *__restrict__ amax,
                      uint32_t slot) {
+    moe_pdl_begin();
     const uint32_t n4 = n / 4u, i0 = blockIdx.x * (EL_THREADS * EL_VECS) + threadIdx.x;
     float4 v[EL_VECS];
 #pragma unroll
@@ -430,13 +436,13 @@ extern "C" void moe_cuda_cast_f16(moe_cuda_ctx_t *c, const float *src, void *dst
     if (pc.n == 0) return;
     if ((uintptr_t)src % 16 == 0 && (uintptr_t)dst % 8 == 0) {
         const uint32_t per = 4u * EL_VECS * EL_THREADS, blocks = (uint32_t)(((uint64_t)pc.n + per - 1u) / per);
-        moe_cast4_f16_kernel<<<blocks, EL_THREADS, 0, c->stream>>>((const float4 *)src, (uint2 *)dst, pc.n, amax, pc.slot);
+        moe_run(c, moe_cast4_f16_kernel, blocks, EL_THREADS, 0, (const float4 *)src, (uint2 *)dst, pc.n, amax, pc.slot);
         MOE_LAUNCHED(c);
         return;
     }
     uint32_t blocks = (uint32_t)(((uint64_t)pc.n + 255u) / 256u);
     if (blocks > (uint32_t)c->sm_count * 16u) blocks = (uint32_t)c->sm_count * 16u;
-    moe_cast_f16_kernel<<<blocks, 256, 0, c->stream>>>(src, (__half *)dst, pc.n, amax, pc.slot);
+    moe_run(c, moe_cast_f16_kernel, blocks, 256, 0, src, (__half *)dst, pc.n, amax, pc.slot);
     MOE_LAUNCHED(c);
 }
 

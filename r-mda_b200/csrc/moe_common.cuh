@@ -112,6 +112,25 @@ bool moe_tmap_gate_up_f16(moe_cuda_ctx *c, CUtensorMap *out, const void *ptr, ui
         }                                                                                 \
     } while (0)
 
+// Launch that may begin while the kernel before it in the stream is still running: the kernel must wait for that one
+// with moe_pdl_begin() before it touches memory.  Launch latency and prologue then hide behind the running kernel (two
+// microseconds per launch).  Under expert parallelism launches stay serial: a kernel that waits there may hold the SMs
+// that another slice's kernel, for which a peer is waiting, still needs.
+template <typename... P, typename... A>
+static inline void moe_run(moe_cuda_ctx *c, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = c->ep == NULL ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // MOE_LAUNCHED looks at the error and counts
+}
+
 // Internal launch helpers shared between the ABI entry points and the fused layer.
 void moe_launch_route(moe_cuda_ctx *c, const float *proj, uint32_t *idx, float *wt, uint32_t *count,
                       uint32_t rows, uint32_t experts, uint32_t topk, uint32_t stride);
@@ -186,6 +205,13 @@ void moe_overlap_prepare_combine(moe_cuda_ctx *c);
 void moe_overlap_prepare_scatter(moe_cuda_ctx *c);
 
 // ---- device helpers -------------------------------------------------------
+// First statement of a kernel launched by moe_run: returns when every kernel before it has completed and its writes are
+// visible; from then on the next one may be set up.
+__device__ __forceinline__ void moe_pdl_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // shader/moe_scan.comp:14-38, for a block of at least 512 threads (all threads of the block must
 // call it; thread e < 512 handles expert e).  count is read past L1.
 __device__ __forceinline__ void moe_scan_body(const uint32_t *count, uint32_t *off, uint32_t *tiles, uint32_t experts,

@@ -18,6 +18,7 @@ __device__ __forceinline__ float dn_sigmoid(float v) { return 1.0f / (1.0f + exp
 // op 1: y = x * scale * rsqrt(sum(x^2) + 1e-6), no weight (:45-61).
 __global__ void __launch_bounds__(NR_THREADS)
 moe_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ y, struct mda_pc_qwen_norm_t pc) {
+    moe_pdl_begin();
     __shared__ float red[NR_THREADS / 32];
     const uint32_t r = blockIdx.x / pc.groups, g = blockIdx.x % pc.groups;
     const float *xi = x + (size_t)r * pc.in_stride + pc.in_off + (size_t)g * pc.in_gstride;
@@ -47,7 +48,7 @@ extern "C" void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w,
     MOE_REQUIRE(c, x != NULL && y != NULL && (w != NULL || pc.op == 1u), "norm: null buffer");
     MOE_REQUIRE(c, pc.groups >= 1 && pc.gsize >= 1, "norm: empty group");
     if (pc.rows == 0) return;
-    moe_norm_kernel<<<pc.rows * pc.groups, NR_THREADS, 0, c->stream>>>(x, w, y, pc);
+    moe_run(c, moe_norm_kernel, pc.rows * pc.groups, NR_THREADS, 0, x, w, y, pc);
     MOE_LAUNCHED(c);
 }
 
@@ -56,6 +57,7 @@ extern "C" void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w,
 // op 2: h[i] += a[i] + b[i]  (:36-38).
 __global__ void moe_hc_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ h,
                               struct mda_pc_qwen_hc_t pc) {
+    moe_pdl_begin();
     const size_t n = (size_t)pc.rows * pc.d * (pc.op == 2u ? pc.hc : 1u);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -86,6 +88,7 @@ __global__ void moe_hc_kernel(const float *__restrict__ a, const float *__restri
 template <uint32_t HC>
 __global__ void __launch_bounds__(NR_THREADS)
 moe_hc_read4_kernel(const float4 *__restrict__ a, const float4 *__restrict__ b, float4 *__restrict__ h, uint32_t total4, uint32_t d4) {
+    moe_pdl_begin();
     const uint32_t i = blockIdx.x * NR_THREADS + threadIdx.x;
     if (i >= total4) return;
     const uint32_t r = i / d4;
@@ -116,14 +119,14 @@ extern "C" void moe_cuda_hc(moe_cuda_ctx_t *c, const float *a, const float *b, f
     // the teacher's four streams; other counts and ragged or unaligned rows take the general form below
     if (pc.op == 0u && pc.hc == 4u && pc.d % 4u == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)h) % 16 == 0 && n / 4 < (1ull << 31)) {
         const uint32_t total4 = (uint32_t)(n / 4);
-        moe_hc_read4_kernel<4><<<(total4 + NR_THREADS - 1u) / NR_THREADS, NR_THREADS, 0, c->stream>>>(
+        moe_run(c, moe_hc_read4_kernel<4>, (total4 + NR_THREADS - 1u) / NR_THREADS, NR_THREADS, 0, 
             (const float4 *)a, (const float4 *)b, (float4 *)h, total4, pc.d / 4u);
         MOE_LAUNCHED(c);
         return;
     }
     size_t blocks = (n + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
-    moe_hc_kernel<<<(unsigned)blocks, 256, 0, c->stream>>>(a, b, h, pc);
+    moe_run(c, moe_hc_kernel, (unsigned)blocks, 256, 0, a, b, h, pc);
     MOE_LAUNCHED(c);
 }
 

@@ -123,6 +123,8 @@ moe_mm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
 
+    moe_pdl_begin();
+
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
@@ -351,7 +353,7 @@ void mm_launch(moe_cuda_ctx *c, const CUtensorMap &tmA, const CUtensorMap &tmB, 
         MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_mm_kernel<MODE, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
         c->mm_attr_set[slot] = true;
     }
-    moe_mm_kernel<MODE, GATHER><<<grid, MM_THREADS + (GATHER ? 128 : 0), MM_SMEM, c->stream>>>(tmA, tmB, a);
+    moe_run(c, moe_mm_kernel<MODE, GATHER>, grid, MM_THREADS + (GATHER ? 128 : 0), MM_SMEM, tmA, tmB, a);
     MOE_LAUNCHED(c);
 }
 

@@ -219,7 +219,6 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
     // feature tiles: SwiGLU 64 outputs (64 gate + 64 up rows) per CTA, otherwise 128 weight rows per CTA
     const uint32_t ft_count = MODE == MOE_MM_SWIGLU_F16 ? (a.n / 2u) / (64u * PAIR) : (a.n + 128u * PAIR - 1u) / (128u * PAIR);
-    const uint32_t total = MODE == MM_DENSE ? (a.rows + a.per - 1u) / a.per * ft_count * a.splits : *a.n_chunks * ft_count;
     const uint32_t kblocks = (a.k + BK - 1) / BK;
     const uint32_t cluster_id = blockIdx.x / PAIR, n_clusters = gridDim.x / PAIR;
 
@@ -252,6 +251,8 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     __syncthreads();
     if (PAIR == 2) cluster_sync_all();  // the peer's barriers exist before anything is sent to them
     tc_fence_after();
+    moe_pdl_begin();
+    const uint32_t total = MODE == MM_DENSE ? (a.rows + a.per - 1u) / a.per * ft_count * a.splits : *a.n_chunks * ft_count;
     const uint32_t tmem_base = bars->tmem_base;
 
     if (warp == 0 || warp >= 6) {
@@ -500,6 +501,7 @@ moe_chunk_kernel(const uint32_t *__restrict__ count, const uint32_t *__restrict_
 // C = the sum of the partial products of a split K, in split order.  n and with it every row is a multiple of four.
 __global__ void __launch_bounds__(256)
 moe_ksum_kernel(const float4 *__restrict__ part, float4 *__restrict__ C, uint32_t total4, uint32_t splits) {
+    moe_pdl_begin();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= total4) return;
     float4 acc = __ldcg(part + i);
@@ -526,13 +528,15 @@ void ws_launch(moe_cuda_ctx *c, const CUtensorMap &tmW, const moe_xmaps &tmX, Ws
     cfg.blockDim = dim3(WS_THREADS, 1, 1);
     cfg.dynamicSmemBytes = ws_smem<PAIR>();
     cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];  // the second as in moe_run
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = PAIR;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = c->ep == NULL ? 2 : 1;
     MOE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, moe_mm_ws_kernel<MODE, PAIR>, tmW, tmX, a));
     c->launches += 1;
 }
@@ -661,7 +665,7 @@ void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C
     ws_launch<MM_DENSE, 2>(c, tmW, tmX, a, (uint32_t)(total < clusters ? total : clusters) * 2u);
     if (a.splits > 1 && MOE_LIVE(c)) {
         const uint32_t total4 = rows * (n / 4u);
-        moe_ksum_kernel<<<(total4 + 255u) / 256u, 256, 0, c->stream>>>((const float4 *)a.C, (float4 *)C, total4, a.splits);
+        moe_run(c, moe_ksum_kernel, (total4 + 255u) / 256u, 256, 0, (const float4 *)a.C, (float4 *)C, total4, a.splits);
         MOE_LAUNCHED(c);
     }
 }

@@ -24,6 +24,7 @@ moe_route_kernel(const float *__restrict__ proj, uint32_t *__restrict__ idx, flo
                  uint32_t *__restrict__ count, uint32_t rows, uint32_t experts, uint32_t topk,
                  uint32_t stride, uint32_t *status, int vec_ok, uint32_t *__restrict__ ones_a, uint32_t n_a,
                  uint32_t *__restrict__ ones_b, uint32_t n_b) {
+    moe_pdl_begin();
     __shared__ uint32_t s_hist[HIST ? MOE_MAX_EXPERTS : 1];
     if (HIST) {
         // the fills of src/qwen.c:796 ride along: tables that later kernels expect to start as ~0
@@ -126,10 +127,10 @@ static void route_dispatch(moe_cuda_ctx *c, uint32_t blocks, const float *proj, 
     const uint32_t nb = (experts + 127u) / 128u;
     const dim3 g(blocks), t(ROUTE_WARPS * 32);
 #define ROUTE_ARGS proj, idx, wt, count, rows, experts, topk, stride, c->dev_status_dev, vec_ok, ones_a, n_a, ones_b, n_b
-    if (nb == 1) moe_route_kernel<HIST, 1><<<g, t, 0, c->stream>>>(ROUTE_ARGS);
-    else if (nb == 2) moe_route_kernel<HIST, 2><<<g, t, 0, c->stream>>>(ROUTE_ARGS);
-    else if (nb == 3) moe_route_kernel<HIST, 3><<<g, t, 0, c->stream>>>(ROUTE_ARGS);
-    else moe_route_kernel<HIST, 4><<<g, t, 0, c->stream>>>(ROUTE_ARGS);
+    if (nb == 1) moe_run(c, moe_route_kernel<HIST, 1>, g, t, 0, ROUTE_ARGS);
+    else if (nb == 2) moe_run(c, moe_route_kernel<HIST, 2>, g, t, 0, ROUTE_ARGS);
+    else if (nb == 3) moe_run(c, moe_route_kernel<HIST, 3>, g, t, 0, ROUTE_ARGS);
+    else moe_run(c, moe_route_kernel<HIST, 4>, g, t, 0, ROUTE_ARGS);
 #undef ROUTE_ARGS
     MOE_LAUNCHED(c);
 }
@@ -175,6 +176,7 @@ extern "C" void moe_cuda_route(moe_cuda_ctx_t *c, const float *proj, uint32_t *i
 __global__ void __launch_bounds__(512)
 moe_scan_kernel(const uint32_t *__restrict__ count, uint32_t *__restrict__ off, uint32_t *__restrict__ tiles,
                 uint32_t experts, uint32_t tile) {
+    moe_pdl_begin();
     moe_scan_body(count, off, tiles, experts, tile);
 }
 
@@ -184,7 +186,7 @@ void moe_launch_scan(moe_cuda_ctx *c, const uint32_t *count, uint32_t *off, uint
     MOE_REQUIRE(c, experts >= 1 && experts <= MOE_MAX_EXPERTS, "scan: experts %u outside 1..512", experts);
     MOE_REQUIRE(c, tile >= 1, "scan: tile 0");
     MOE_REQUIRE(c, count != NULL && off != NULL && tiles != NULL, "scan: null buffer");
-    moe_scan_kernel<<<1, 512, 0, c->stream>>>(count, off, tiles, experts, tile);
+    moe_run(c, moe_scan_kernel, 1, 512, 0, count, off, tiles, experts, tile);
     MOE_LAUNCHED(c);
 }
 

@@ -19,6 +19,7 @@
 __global__ void __launch_bounds__(SC_PAIRS)
 moe_scatter_hist_kernel(const uint32_t *__restrict__ idx, uint32_t *__restrict__ hist, uint32_t pairs,
                         uint32_t ebound, uint32_t *status) {
+    moe_pdl_begin();
     extern __shared__ uint32_t sh[];
     for (uint32_t e = threadIdx.x; e < ebound; e += SC_PAIRS) sh[e] = 0;
     __syncthreads();
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(1024)
 moe_scatter_colscan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ fill, uint32_t nblocks,
                            uint32_t ebound, uint32_t *__restrict__ count_out, uint32_t *ticket, uint32_t *off,
                            uint32_t *tiles, uint32_t tile, uint4 *chunks, uint32_t *n_chunks, uint32_t max_chunks) {
+    moe_pdl_begin();
     __shared__ uint32_t seg_sum[32][33];
     __shared__ uint32_t s_last;
     uint32_t el = threadIdx.x & 31u, seg = threadIdx.x >> 5;
@@ -119,6 +121,7 @@ moe_scatter_place_kernel(const uint32_t *__restrict__ idx, const uint32_t *__res
                          uint32_t d8, uint32_t ebound, uint4 *const *__restrict__ xp_peers, uint32_t experts_per_rank,
                          uint32_t ppb, uint32_t *__restrict__ src_row, uint32_t *const *__restrict__ src_row_peers,
                          uint32_t src_base, uint2 *const *__restrict__ ret_peers, const float *__restrict__ wt) {
+    moe_pdl_begin();
     // ppb = pairs per block (<= SC_MAX_PAIRS): 64 in the stand-alone scatter, 8*topk behind the fused router.
     // A block takes pair groups blockIdx.x, blockIdx.x + gridDim.x, ...; the gridDim.y blocks of a group share its
     // row copies (sc_copy_split): each ranks all pairs, the first writes the tables.
@@ -210,14 +213,14 @@ void moe_launch_scatter(moe_cuda_ctx *c, const uint32_t *idx, const uint32_t *of
     uint32_t nblocks = (pairs + SC_PAIRS - 1) / SC_PAIRS;
     uint32_t *hist = (uint32_t *)moe_scratch(c, MOE_SCR_SCATTER, (size_t)nblocks * ebound * sizeof(uint32_t));
     if (hist == NULL) return;
-    moe_scatter_hist_kernel<<<nblocks, SC_PAIRS, ebound * sizeof(uint32_t), c->stream>>>(idx, hist, pairs, ebound,
+    moe_run(c, moe_scatter_hist_kernel, nblocks, SC_PAIRS, ebound * sizeof(uint32_t), idx, hist, pairs, ebound,
                                                                                          c->dev_status_dev);
     MOE_LAUNCHED(c);
-    moe_scatter_colscan_kernel<<<(ebound + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, c->stream>>>(hist, fill, nblocks, ebound, NULL, NULL, NULL, NULL, 0, NULL, NULL, 0);
+    moe_run(c, moe_scatter_colscan_kernel, (ebound + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, fill, nblocks, ebound, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
     MOE_LAUNCHED(c);
-    moe_scatter_place_kernel<<<dim3(nblocks, sc_copy_split(c, nblocks, SC_PAIRS)), SC_THREADS, 0, c->stream>>>(idx, off, hist, (const uint4 *)x16, (uint4 *)xp,
+    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, sc_copy_split(c, nblocks, SC_PAIRS)), SC_THREADS, 0, idx, off, hist, (const uint4 *)x16, (uint4 *)xp,
                                                                     slot, pairs, topk, d8, ebound,
-                                                                    (uint4 *const *)xp_peers, experts_per_rank, SC_PAIRS, NULL, NULL, 0, NULL, NULL);
+                                                                    (uint4 *const *)xp_peers, experts_per_rank, SC_PAIRS, nullptr, nullptr, 0, nullptr, nullptr);
     MOE_LAUNCHED(c);
 }
 
@@ -238,7 +241,7 @@ void moe_launch_colscan_counts(moe_cuda_ctx *c, uint32_t *hist, uint32_t *count,
         }
         ticket = c->ticket;
     }
-    moe_scatter_colscan_kernel<<<(experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, c->stream>>>(hist, NULL, nblocks, experts, count,
+    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, nullptr, nblocks, experts, count,
                                                                                                  ticket, off, tiles, tile,
                                                                                                  (uint4 *)chunks, n_chunks, max_chunks);
     MOE_LAUNCHED(c);
@@ -262,7 +265,7 @@ void moe_launch_place(moe_cuda_ctx *c, const uint32_t *idx, const uint32_t *off,
     uint32_t nblocks = (rows + 7u) / 8u;
     // gather modes copy nothing
     const uint32_t split = src_row == NULL && src_row_peers == NULL ? sc_copy_split(c, nblocks, 8u * topk) : 1u;
-    moe_scatter_place_kernel<<<dim3(nblocks, split), SC_THREADS, 0, c->stream>>>(idx, off, hist, (const uint4 *)x16, (uint4 *)xp, slot,
+    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, split), SC_THREADS, 0, idx, off, hist, (const uint4 *)x16, (uint4 *)xp, slot,
                                                                     rows * topk, topk, d8, experts,
                                                                     (uint4 *const *)xp_peers, experts_per_rank, 8u * topk, src_row,
                                                                     src_row_peers, src_base, ret_peers, wt);
@@ -322,12 +325,12 @@ extern "C" void moe_cuda_scatter_noalloc(moe_cuda_ctx_t *c, const uint32_t *idx,
     if (pairs == 0) return;
     // The table keeps the previous call's contents; nothing has to start at zero
     // because the hist kernel writes every entry the later kernels read.
-    moe_scatter_hist_kernel<<<(uint32_t)nblocks, SC_PAIRS, experts * sizeof(uint32_t), c->stream>>>(
+    moe_run(c, moe_scatter_hist_kernel, (uint32_t)nblocks, SC_PAIRS, experts * sizeof(uint32_t), 
         idx, table, (uint32_t)pairs, experts, c->dev_status_dev);
     MOE_LAUNCHED(c);
-    moe_scatter_colscan_kernel<<<(experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, c->stream>>>(table, fill, (uint32_t)nblocks, experts, NULL, NULL, NULL, NULL, 0, NULL, NULL, 0);
+    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, table, fill, (uint32_t)nblocks, experts, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
     MOE_LAUNCHED(c);
-    moe_scatter_place_kernel<<<dim3((uint32_t)nblocks, sc_copy_split(c, (uint32_t)nblocks, SC_PAIRS)), SC_THREADS, 0, c->stream>>>(
-        idx, off, table, (const uint4 *)x16, (uint4 *)xp, slot, (uint32_t)pairs, pc.topk, pc.d8, experts, NULL, 0, SC_PAIRS, NULL, NULL, 0, NULL, NULL);
+    moe_run(c, moe_scatter_place_kernel, dim3((uint32_t)nblocks, sc_copy_split(c, (uint32_t)nblocks, SC_PAIRS)), SC_THREADS, 0, 
+        idx, off, table, (const uint4 *)x16, (uint4 *)xp, slot, (uint32_t)pairs, pc.topk, pc.d8, experts, nullptr, 0, SC_PAIRS, nullptr, nullptr, 0, nullptr, nullptr);
     MOE_LAUNCHED(c);
 }
