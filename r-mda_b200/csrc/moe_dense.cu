@@ -40,6 +40,44 @@ moe_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float 
     }
 }
 
+// The same with groups of at most NR_THREADS * 4 * NV columns, all on 16 bytes: the group is read once and kept in
+// registers.  Bound by HBM; 3001 rows of 4 x 2048: 36.6 us read twice in single values, 34.0 us this way.
+template <int NV>
+__global__ void __launch_bounds__(NR_THREADS)
+moe_norm4_kernel(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ y, struct mda_pc_qwen_norm_t pc) {
+    moe_pdl_begin();
+    __shared__ float red[NR_THREADS / 32];
+    const uint32_t r = blockIdx.x / pc.groups, g = blockIdx.x % pc.groups, n4 = pc.gsize / 4u;
+    const float4 *xi = reinterpret_cast<const float4 *>(x + (size_t)r * pc.in_stride + pc.in_off + (size_t)g * pc.in_gstride);
+    float4 *yi = reinterpret_cast<float4 *>(y + (size_t)r * pc.out_stride + pc.out_off + (size_t)g * pc.out_gstride);
+    const bool weighted = pc.op == 0u && w != NULL;
+    const float4 *wi = weighted ? reinterpret_cast<const float4 *>(w + pc.w_off + (size_t)g * pc.wstride) : NULL;
+    float4 v[NV], wv[NV];
+    float acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NV; i += 1) {
+        const uint32_t c = i * NR_THREADS + threadIdx.x;
+        v[i] = c < n4 ? xi[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+        wv[i] = weighted && c < n4 ? __ldg(wi + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i += 1) acc += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    float ss = 0.0f;
+#pragma unroll
+    for (uint32_t q = 0; q < NR_THREADS / 32; q += 1) ss += red[q];
+    const float f = pc.op == 1u ? pc.scale * rsqrtf(ss + 1e-6f) : rsqrtf(ss / (float)pc.gsize + pc.eps);
+#pragma unroll
+    for (int i = 0; i < NV; i += 1) {
+        const uint32_t c = i * NR_THREADS + threadIdx.x;
+        if (c < n4) yi[c] = make_float4(v[i].x * f * (1.0f + wv[i].x), v[i].y * f * (1.0f + wv[i].y),
+                                        v[i].z * f * (1.0f + wv[i].z), v[i].w * f * (1.0f + wv[i].w));
+    }
+}
+
 extern "C" void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w, float *y, const float *z,
                               struct mda_pc_qwen_norm_t pc) {
     (void)z;  // binding 3 of the shader: only its op 2 reads it
@@ -48,6 +86,14 @@ extern "C" void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w,
     MOE_REQUIRE(c, x != NULL && y != NULL && (w != NULL || pc.op == 1u), "norm: null buffer");
     MOE_REQUIRE(c, pc.groups >= 1 && pc.gsize >= 1, "norm: empty group");
     if (pc.rows == 0) return;
+    const uint32_t wlay = pc.op == 0u ? pc.w_off | pc.wstride : 0u;
+    if ((pc.gsize | pc.in_stride | pc.in_off | pc.in_gstride | pc.out_stride | pc.out_off | pc.out_gstride | wlay) % 4u == 0 &&
+        (((uintptr_t)x | (uintptr_t)y | (pc.op == 0u ? (uintptr_t)w : 0u)) & 15) == 0 && pc.gsize <= NR_THREADS * 4u * 4u) {
+        if (pc.gsize <= NR_THREADS * 4u * 2u) moe_run(c, moe_norm4_kernel<2>, pc.rows * pc.groups, NR_THREADS, 0, x, w, y, pc);
+        else moe_run(c, moe_norm4_kernel<4>, pc.rows * pc.groups, NR_THREADS, 0, x, w, y, pc);
+        MOE_LAUNCHED(c);
+        return;
+    }
     moe_run(c, moe_norm_kernel, pc.rows * pc.groups, NR_THREADS, 0, x, w, y, pc);
     MOE_LAUNCHED(c);
 }
