@@ -327,6 +327,40 @@ def test_kd_bytes_edges(ctx, oracle, rows, vocab, alphabet, lift):
     assert ((got & 0xffff) != (ref & 0xffff)).mean() < 0.01
 
 
+@pytest.mark.parametrize("rows,vocab", [(16, 5003), (1280, 20000)])   # one chunk per block of the sweep; four
+def test_kd_bytes_special_logits(ctx, oracle, rows, vocab):
+    """Rows masked in part or whole, without any finite logit, with NaN, infinities or a logit so large that small
+    differences from it vanish: the oracle's result, not a number or infinite where it is."""
+    rng = np.random.default_rng(vocab)
+    length = rng.integers(0, 7, vocab)
+    tb = rng.integers(97, 123, (vocab, 16)).astype(np.uint8)
+    tb[np.arange(16)[None, :] >= length[:, None]] = 0
+    toks = np.ascontiguousarray(np.concatenate([tb.view(np.uint32).reshape(vocab, 4), length[:, None].astype(np.uint32)], 1))
+    cont = np.zeros((rows, 5), np.uint32)
+    cont[:, :4] = rng.integers(97, 123, (rows, 16)).astype(np.uint8).view(np.uint32).reshape(rows, 4)
+    cont[:, 4] = 3
+    logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
+    half, inf, nan, low = vocab // 2, np.inf, np.nan, np.finfo(np.float32).min
+    spoiled = [(slice(None), -inf), (slice(None), low), (slice(None), -3.0e38), (slice(None), -1e38), (slice(0, half), -inf),
+               (slice(half, None), -inf), (slice(0, None, 2), -inf), (77, nan), (vocab - 80, nan), (slice(None), nan), (100, inf),
+               (vocab - 100, inf), (slice(0, 100), inf), (5, 1e38), (vocab - 5, 1e10)]
+    for r, (where, value) in enumerate(spoiled):
+        logits[r * (rows // 16), where] = value
+    logits[-1] = -inf
+    logits[-1, 3], logits[-1, vocab - 4] = 5.0, nan
+    d_out = ctx.alloc(rows * 16 * 8 * 4).fill(0xdeadbeef)
+    ctx.kd_bytes(ctx.upload(logits), ctx.upload(toks), ctx.upload(cont), d_out, rows, vocab)
+    ctx.flush()
+    got, ref = d_out.read(np.uint32, (rows, 16, 8)), oracle.kd_bytes(logits, toks, cont)
+    pg = (got >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    pr = (ref >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    finite = np.isfinite(pr)
+    assert np.array_equal(pg[~finite], pr[~finite], equal_nan=True)
+    assert np.all(np.abs(pg - pr)[finite] <= 1.5e-3 * pr[finite] + 1e-7)
+    assert np.array_equal(got[..., 0] & 0xffff, ref[..., 0] & 0xffff)
+    assert ((got & 0xffff) != (ref & 0xffff)).mean() < 0.01
+
+
 def test_fill_and_copy(ctx):
     b = ctx.alloc(4 * 1003)
     b.fill(0x12345678)
