@@ -18,7 +18,7 @@ template <> struct moe_vec<__half, 4> { typedef uint2 raw; };
 template <> struct moe_vec<__half, 8> { typedef uint4 raw; };
 template <typename YT, int V>
 __device__ __forceinline__ typename moe_vec<YT, V>::raw moe_fetch(const YT *p) {
-    return __ldg(reinterpret_cast<const typename moe_vec<YT, V>::raw *>(p));
+    return *reinterpret_cast<const typename moe_vec<YT, V>::raw *>(p);
 }
 __device__ __forceinline__ void moe_floats(float4 r, float (&f)[4]) {
     f[0] = r.x; f[1] = r.y; f[2] = r.z; f[3] = r.w;
@@ -130,7 +130,7 @@ moe_combine_kernel(moe_combine_args a) {
                 if (a.sh != NULL) {
 #pragma unroll
                     for (int i = 0; i < V; i += 4) {
-                        const float4 v = __ldg(reinterpret_cast<const float4 *>(a.sh + (size_t)r * a.d + c + i));
+                        const float4 v = *reinterpret_cast<const float4 *>(a.sh + (size_t)r * a.d + c + i);
                         acc[i] = __fadd_rn(acc[i], __fmul_rn(sg, v.x));
                         acc[i + 1] = __fadd_rn(acc[i + 1], __fmul_rn(sg, v.y));
                         acc[i + 2] = __fadd_rn(acc[i + 2], __fmul_rn(sg, v.z));
@@ -284,7 +284,7 @@ __device__ __forceinline__ float moe_elem(float g, float u, uint32_t op, float s
 }
 
 // General form: any n, stride, offset and alignment.
-__global__ void moe_swiglu_kernel(const float *__restrict__ a, float *__restrict__ y, uint32_t rows, uint32_t n,
+__global__ void moe_swiglu_kernel(const float *a, float *__restrict__ y, uint32_t rows, uint32_t n,
                                   uint32_t astride, uint32_t ao, uint32_t bo, uint32_t op, float scale) {
     moe_pdl_begin();
     size_t total = (size_t)rows * n;
@@ -299,7 +299,7 @@ __global__ void moe_swiglu_kernel(const float *__restrict__ a, float *__restrict
 // Rows, offsets and strides in whole float4: total4 = rows * n4 values of four, below 2^31.
 template <uint32_t OP>
 __global__ void __launch_bounds__(EL_THREADS)
-moe_swiglu4_kernel(const float4 *__restrict__ a, float4 *__restrict__ y, uint32_t total4, uint32_t n4, uint32_t astride4,
+moe_swiglu4_kernel(const float4 *a, float4 *__restrict__ y, uint32_t total4, uint32_t n4, uint32_t astride4,
                    uint32_t ao4, uint32_t bo4, float scale) {
     moe_pdl_begin();
     constexpr uint32_t U = 2;  // two operands: four loads in flight
@@ -311,8 +311,8 @@ moe_swiglu4_kernel(const float4 *__restrict__ a, float4 *__restrict__ y, uint32_
         if (i >= total4) break;
         const uint32_t r = i / n4;
         const float4 *row = a + (size_t)r * astride4 + (i - r * n4);
-        g[j] = __ldg(row + ao4);
-        u[j] = OP == 0u ? __ldg(row + bo4) : g[j];
+        g[j] = row[ao4];
+        u[j] = OP == 0u ? row[bo4] : g[j];
     }
 #pragma unroll
     for (uint32_t j = 0; j < U; j += 1) {
@@ -350,7 +350,7 @@ extern "C" void moe_cuda_swiglu(moe_cuda_ctx_t *c, const float *a, float *y, str
 
 // n4 float4 from the first 16-byte boundary of x on; the few values before and behind them go to the first threads.
 __global__ void __launch_bounds__(EL_THREADS)
-moe_absmax_kernel(const float *__restrict__ x, uint32_t *__restrict__ amax, uint32_t n, uint32_t head, uint32_t slot) {
+moe_absmax_kernel(const float *x, uint32_t *__restrict__ amax, uint32_t n, uint32_t head, uint32_t slot) {
     moe_pdl_begin();
     __shared__ float red[EL_THREADS / 32];
     const uint32_t n4 = (n - head) / 4u, stride = gridDim.x * EL_THREADS;
@@ -361,7 +361,7 @@ moe_absmax_kernel(const float *__restrict__ x, uint32_t *__restrict__ amax, uint
         float4 v[EL_VECS];
 #pragma unroll
         for (uint32_t j = 0; j < EL_VECS; j += 1) {
-            v[j] = base + j * stride < n4 ? __ldg(x4 + base + j * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[j] = base + j * stride < n4 ? x4[base + j * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (uint32_t j = 0; j < EL_VECS; j += 1) {
@@ -399,8 +399,8 @@ __device__ __forceinline__ uint2 moe_pack4(float4 v, float s) {
 }
 
 // General form: any alignment.
-__global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__restrict__ dst, size_t n,
-                                    const uint32_t *__restrict__ amax, uint32_t slot) {
+__global__ void moe_cast_f16_kernel(const float *src, __half *__restrict__ dst, size_t n, const uint32_t *amax,
+                                    uint32_t slot) {
     moe_pdl_begin();
     float s = moe_slot_scale(amax, slot);
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -411,14 +411,14 @@ __global__ void moe_cast_f16_kernel(const float *__restrict__ src, __half *__res
 
 // src on 16 bytes, dst on 8.
 __global__ void __launch_bounds__(EL_THREADS)
-moe_cast4_f16_kernel(const float4 *__restrict__ src, uint2 *__restrict__ dst, uint32_t n, const uint32_t *__restrict__ amax,
+moe_cast4_f16_kernel(const float4 *src, uint2 *__restrict__ dst, uint32_t n, const uint32_t *amax,
                      uint32_t slot) {
     moe_pdl_begin();
     const uint32_t n4 = n / 4u, i0 = blockIdx.x * (EL_THREADS * EL_VECS) + threadIdx.x;
     float4 v[EL_VECS];
 #pragma unroll
     for (uint32_t j = 0; j < EL_VECS; j += 1) {
-        if (i0 + j * EL_THREADS < n4) v[j] = __ldg(src + i0 + j * EL_THREADS);
+        if (i0 + j * EL_THREADS < n4) v[j] = src[i0 + j * EL_THREADS];
     }
     const float s = moe_slot_scale(amax, slot);
 #pragma unroll

@@ -20,7 +20,7 @@
 // NB = ceil(experts / 128): how many 128-expert blocks each lane really holds.
 template <bool HIST, int NB>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_kernel(const float *__restrict__ proj, uint32_t *__restrict__ idx, float *__restrict__ wt,
+moe_route_kernel(const float *proj, uint32_t *__restrict__ idx, float *__restrict__ wt,
                  uint32_t *__restrict__ count, uint32_t rows, uint32_t experts, uint32_t topk,
                  uint32_t stride, uint32_t *status, int vec_ok, uint32_t *__restrict__ ones_a, uint32_t n_a,
                  uint32_t *__restrict__ ones_b, uint32_t n_b) {
@@ -45,7 +45,7 @@ moe_route_kernel(const float *__restrict__ proj, uint32_t *__restrict__ idx, flo
         for (uint32_t j = 0; j < NB; j += 1) {
             uint32_t e0 = 4u * lane + 128u * j;
             if (vec_ok && e0 + 3u < experts) {
-                float4 v = __ldg(reinterpret_cast<const float4 *>(row + e0));
+                float4 v = *reinterpret_cast<const float4 *>(row + e0);
                 l[4 * j + 0] = v.x;
                 l[4 * j + 1] = v.y;
                 l[4 * j + 2] = v.z;
@@ -53,7 +53,7 @@ moe_route_kernel(const float *__restrict__ proj, uint32_t *__restrict__ idx, flo
             } else {
 #pragma unroll
                 for (uint32_t q = 0; q < 4; q += 1) {
-                    l[4 * j + q] = e0 + q < experts ? __ldg(row + e0 + q) : ROUTE_SENTINEL;
+                    l[4 * j + q] = e0 + q < experts ? row[e0 + q] : ROUTE_SENTINEL;
                 }
             }
         }
@@ -174,7 +174,7 @@ extern "C" void moe_cuda_route(moe_cuda_ctx_t *c, const float *proj, uint32_t *i
 // shader/moe_scan.comp:14-38: one 512-thread block; pad each count to the tile,
 // exclusive prefix sum, one tiles[] entry per padded tile (moe_scan_body, moe_common.cuh).
 __global__ void __launch_bounds__(512)
-moe_scan_kernel(const uint32_t *__restrict__ count, uint32_t *__restrict__ off, uint32_t *__restrict__ tiles,
+moe_scan_kernel(const uint32_t *count, uint32_t *__restrict__ off, uint32_t *__restrict__ tiles,
                 uint32_t experts, uint32_t tile) {
     moe_pdl_begin();
     moe_scan_body(count, off, tiles, experts, tile);

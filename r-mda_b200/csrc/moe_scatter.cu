@@ -17,7 +17,7 @@
 #define SC_THREADS 256u
 
 __global__ void __launch_bounds__(SC_PAIRS)
-moe_scatter_hist_kernel(const uint32_t *__restrict__ idx, uint32_t *__restrict__ hist, uint32_t pairs,
+moe_scatter_hist_kernel(const uint32_t *idx, uint32_t *__restrict__ hist, uint32_t pairs,
                         uint32_t ebound, uint32_t *status) {
     moe_pdl_begin();
     extern __shared__ uint32_t sh[];
@@ -115,12 +115,11 @@ moe_scatter_colscan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ f
 }
 
 __global__ void __launch_bounds__(SC_THREADS)
-moe_scatter_place_kernel(const uint32_t *__restrict__ idx, const uint32_t *__restrict__ off,
-                         const uint32_t *__restrict__ base, const uint4 *__restrict__ x16,
+moe_scatter_place_kernel(const uint32_t *idx, const uint32_t *off, const uint32_t *base, const uint4 *x16,
                          uint4 *__restrict__ xp, uint32_t *__restrict__ slot, uint32_t pairs, uint32_t topk,
-                         uint32_t d8, uint32_t ebound, uint4 *const *__restrict__ xp_peers, uint32_t experts_per_rank,
-                         uint32_t ppb, uint32_t *__restrict__ src_row, uint32_t *const *__restrict__ src_row_peers,
-                         uint32_t src_base, uint2 *const *__restrict__ ret_peers, const float *__restrict__ wt) {
+                         uint32_t d8, uint32_t ebound, uint4 *const *xp_peers, uint32_t experts_per_rank,
+                         uint32_t ppb, uint32_t *__restrict__ src_row, uint32_t *const *src_row_peers,
+                         uint32_t src_base, uint2 *const *ret_peers, const float *wt) {
     moe_pdl_begin();
     // ppb = pairs per block (<= SC_MAX_PAIRS): 64 in the stand-alone scatter, 8*topk behind the fused router.
     // A block takes pair groups blockIdx.x, blockIdx.x + gridDim.x, ...; the gridDim.y blocks of a group share its
@@ -178,13 +177,13 @@ moe_scatter_place_kernel(const uint32_t *__restrict__ idx, const uint32_t *__res
                 uint4 *dst = s_dst[q] + (size_t)p * d8;
                 uint32_t i = lane;
                 for (; i + 96u < d8; i += 128u) {  // four 16-byte loads in flight per lane
-                    uint4 a = __ldg(src + i), b = __ldg(src + i + 32u), c2 = __ldg(src + i + 64u), d2 = __ldg(src + i + 96u);
+                    const uint4 a = src[i], b = src[i + 32u], c2 = src[i + 64u], d2 = src[i + 96u];
                     dst[i] = a;
                     dst[i + 32u] = b;
                     dst[i + 64u] = c2;
                     dst[i + 96u] = d2;
                 }
-                for (; i < d8; i += 32u) dst[i] = __ldg(src + i);  // :30-32
+                for (; i < d8; i += 32u) dst[i] = src[i];  // :30-32
             }
             __syncthreads();  // the tables are rewritten by the next group
         }
