@@ -284,7 +284,7 @@ __device__ __forceinline__ float moe_elem(float g, float u, uint32_t op, float s
 }
 
 // General form: any n, stride, offset and alignment.
-__global__ void moe_swiglu_kernel(const float *a, float *__restrict__ y, uint32_t rows, uint32_t n,
+__global__ void moe_swiglu_kernel(const float *a, float *y, uint32_t rows, uint32_t n,
                                   uint32_t astride, uint32_t ao, uint32_t bo, uint32_t op, float scale) {
     moe_pdl_begin();
     size_t total = (size_t)rows * n;
@@ -299,7 +299,7 @@ __global__ void moe_swiglu_kernel(const float *a, float *__restrict__ y, uint32_
 // Rows, offsets and strides in whole float4: total4 = rows * n4 values of four, below 2^31.
 template <uint32_t OP>
 __global__ void __launch_bounds__(EL_THREADS)
-moe_swiglu4_kernel(const float4 *a, float4 *__restrict__ y, uint32_t total4, uint32_t n4, uint32_t astride4,
+moe_swiglu4_kernel(const float4 *a, float4 *y, uint32_t total4, uint32_t n4, uint32_t astride4,
                    uint32_t ao4, uint32_t bo4, float scale) {
     moe_pdl_begin();
     constexpr uint32_t U = 2;  // two operands: four loads in flight
@@ -350,7 +350,7 @@ extern "C" void moe_cuda_swiglu(moe_cuda_ctx_t *c, const float *a, float *y, str
 
 // n4 float4 from the first 16-byte boundary of x on; the few values before and behind them go to the first threads.
 __global__ void __launch_bounds__(EL_THREADS)
-moe_absmax_kernel(const float *x, uint32_t *__restrict__ amax, uint32_t n, uint32_t head, uint32_t slot) {
+moe_absmax_kernel(const float *x, uint32_t *amax, uint32_t n, uint32_t head, uint32_t slot) {
     moe_pdl_begin();
     __shared__ float red[EL_THREADS / 32];
     const uint32_t n4 = (n - head) / 4u, stride = gridDim.x * EL_THREADS;
@@ -399,7 +399,7 @@ __device__ __forceinline__ uint2 moe_pack4(float4 v, float s) {
 }
 
 // General form: any alignment.
-__global__ void moe_cast_f16_kernel(const float *src, __half *__restrict__ dst, size_t n, const uint32_t *amax,
+__global__ void moe_cast_f16_kernel(const float *src, __half *dst, size_t n, const uint32_t *amax,
                                     uint32_t slot) {
     moe_pdl_begin();
     float s = moe_slot_scale(amax, slot);
@@ -411,7 +411,7 @@ __global__ void moe_cast_f16_kernel(const float *src, __half *__restrict__ dst, 
 
 // src on 16 bytes, dst on 8.
 __global__ void __launch_bounds__(EL_THREADS)
-moe_cast4_f16_kernel(const float4 *src, uint2 *__restrict__ dst, uint32_t n, const uint32_t *amax,
+moe_cast4_f16_kernel(const float4 *src, uint2 *dst, uint32_t n, const uint32_t *amax,
                      uint32_t slot) {
     moe_pdl_begin();
     const uint32_t n4 = n / 4u, i0 = blockIdx.x * (EL_THREADS * EL_VECS) + threadIdx.x;

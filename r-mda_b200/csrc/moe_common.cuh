@@ -207,7 +207,8 @@ void moe_overlap_prepare_scatter(moe_cuda_ctx *c);
 // ---- device helpers -------------------------------------------------------
 // First statement of a kernel launched by moe_run: returns when every kernel before it has completed and its writes are
 // visible; from then on the next one may be set up.  The kernel's lifetime has begun before those writes: its inputs are
-// read with plain loads (no __ldg, no const __restrict__ parameters), which cannot be moved in front of the wait.
+// read with plain loads, and no parameter is __restrict__: loads that are promised constant data, and accesses through a
+// pointer that nothing else is said to alias, may be moved in front of the wait.
 __device__ __forceinline__ void moe_pdl_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

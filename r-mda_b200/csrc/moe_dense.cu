@@ -17,7 +17,7 @@ __device__ __forceinline__ float dn_sigmoid(float v) { return 1.0f / (1.0f + exp
 // One block per (row, group), as the shader (:64-67).  op 0: y = x * rsqrt(mean(x^2) + eps) * (1 + w);
 // op 1: y = x * scale * rsqrt(sum(x^2) + 1e-6), no weight (:45-61).
 __global__ void __launch_bounds__(NR_THREADS)
-moe_norm_kernel(const float *x, const float *w, float *__restrict__ y, struct mda_pc_qwen_norm_t pc) {
+moe_norm_kernel(const float *x, const float *w, float *y, struct mda_pc_qwen_norm_t pc) {
     moe_pdl_begin();
     __shared__ float red[NR_THREADS / 32];
     const uint32_t r = blockIdx.x / pc.groups, g = blockIdx.x % pc.groups;
@@ -44,7 +44,7 @@ moe_norm_kernel(const float *x, const float *w, float *__restrict__ y, struct md
 // registers.  Bound by HBM; 3001 rows of 4 x 2048: 36.6 us read twice in single values, 34.0 us this way.
 template <int NV>
 __global__ void __launch_bounds__(NR_THREADS)
-moe_norm4_kernel(const float *x, const float *w, float *__restrict__ y, struct mda_pc_qwen_norm_t pc) {
+moe_norm4_kernel(const float *x, const float *w, float *y, struct mda_pc_qwen_norm_t pc) {
     moe_pdl_begin();
     __shared__ float red[NR_THREADS / 32];
     const uint32_t r = blockIdx.x / pc.groups, g = blockIdx.x % pc.groups, n4 = pc.gsize / 4u;
@@ -101,7 +101,7 @@ extern "C" void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w,
 // shader/qwen_hc.comp.  op 0: h[r,c] = mean_s sigmoid(a[r,s,c]) * b[r,s,c]  (the mixer's read-out, :24-30);
 // op 1: h[r,s,c] += a[r,c] * 2*sigmoid(b[r*inj_stride + inj_off + s] / hc)  (:31-35);
 // op 2: h[i] += a[i] + b[i]  (:36-38).
-__global__ void moe_hc_kernel(const float *a, const float *b, float *__restrict__ h,
+__global__ void moe_hc_kernel(const float *a, const float *b, float *h,
                               struct mda_pc_qwen_hc_t pc) {
     moe_pdl_begin();
     const size_t n = (size_t)pc.rows * pc.d * (pc.op == 2u ? pc.hc : 1u);
@@ -133,7 +133,7 @@ __global__ void moe_hc_kernel(const float *a, const float *b, float *__restrict_
 // together.  Bound by HBM; 3001 rows of 4 x 2048: 76 us one column at a time, 35 us this way.
 template <uint32_t HC>
 __global__ void __launch_bounds__(NR_THREADS)
-moe_hc_read4_kernel(const float4 *a, const float4 *b, float4 *__restrict__ h, uint32_t total4, uint32_t d4) {
+moe_hc_read4_kernel(const float4 *a, const float4 *b, float4 *h, uint32_t total4, uint32_t d4) {
     moe_pdl_begin();
     const uint32_t i = blockIdx.x * NR_THREADS + threadIdx.x;
     if (i >= total4) return;

@@ -500,7 +500,7 @@ moe_chunk_kernel(const uint32_t *__restrict__ count, const uint32_t *__restrict_
 
 // C = the sum of the partial products of a split K, in split order.  n and with it every row is a multiple of four.
 __global__ void __launch_bounds__(256)
-moe_ksum_kernel(const float4 *part, float4 *__restrict__ C, uint32_t total4, uint32_t splits) {
+moe_ksum_kernel(const float4 *part, float4 *C, uint32_t total4, uint32_t splits) {
     moe_pdl_begin();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= total4) return;

@@ -20,10 +20,10 @@
 // NB = ceil(experts / 128): how many 128-expert blocks each lane really holds.
 template <bool HIST, int NB>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_kernel(const float *proj, uint32_t *__restrict__ idx, float *__restrict__ wt,
-                 uint32_t *__restrict__ count, uint32_t rows, uint32_t experts, uint32_t topk,
-                 uint32_t stride, uint32_t *status, int vec_ok, uint32_t *__restrict__ ones_a, uint32_t n_a,
-                 uint32_t *__restrict__ ones_b, uint32_t n_b) {
+moe_route_kernel(const float *proj, uint32_t *idx, float *wt,
+                 uint32_t *count, uint32_t rows, uint32_t experts, uint32_t topk,
+                 uint32_t stride, uint32_t *status, int vec_ok, uint32_t *ones_a, uint32_t n_a,
+                 uint32_t *ones_b, uint32_t n_b) {
     moe_pdl_begin();
     __shared__ uint32_t s_hist[HIST ? MOE_MAX_EXPERTS : 1];
     if (HIST) {
@@ -174,7 +174,7 @@ extern "C" void moe_cuda_route(moe_cuda_ctx_t *c, const float *proj, uint32_t *i
 // shader/moe_scan.comp:14-38: one 512-thread block; pad each count to the tile,
 // exclusive prefix sum, one tiles[] entry per padded tile (moe_scan_body, moe_common.cuh).
 __global__ void __launch_bounds__(512)
-moe_scan_kernel(const uint32_t *count, uint32_t *__restrict__ off, uint32_t *__restrict__ tiles,
+moe_scan_kernel(const uint32_t *count, uint32_t *off, uint32_t *tiles,
                 uint32_t experts, uint32_t tile) {
     moe_pdl_begin();
     moe_scan_body(count, off, tiles, experts, tile);

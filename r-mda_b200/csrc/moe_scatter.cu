@@ -17,7 +17,7 @@
 #define SC_THREADS 256u
 
 __global__ void __launch_bounds__(SC_PAIRS)
-moe_scatter_hist_kernel(const uint32_t *idx, uint32_t *__restrict__ hist, uint32_t pairs,
+moe_scatter_hist_kernel(const uint32_t *idx, uint32_t *hist, uint32_t pairs,
                         uint32_t ebound, uint32_t *status) {
     moe_pdl_begin();
     extern __shared__ uint32_t sh[];
@@ -43,8 +43,8 @@ moe_scatter_hist_kernel(const uint32_t *idx, uint32_t *__restrict__ hist, uint32
 // count_out[e] receives it.
 #define CS_EXPERTS 32u
 __global__ void __launch_bounds__(1024)
-moe_scatter_colscan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ fill, uint32_t nblocks,
-                           uint32_t ebound, uint32_t *__restrict__ count_out, uint32_t *ticket, uint32_t *off,
+moe_scatter_colscan_kernel(uint32_t *hist, uint32_t *fill, uint32_t nblocks,
+                           uint32_t ebound, uint32_t *count_out, uint32_t *ticket, uint32_t *off,
                            uint32_t *tiles, uint32_t tile, uint4 *chunks, uint32_t *n_chunks, uint32_t max_chunks) {
     moe_pdl_begin();
     __shared__ uint32_t seg_sum[32][33];
@@ -116,9 +116,9 @@ moe_scatter_colscan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ f
 
 __global__ void __launch_bounds__(SC_THREADS)
 moe_scatter_place_kernel(const uint32_t *idx, const uint32_t *off, const uint32_t *base, const uint4 *x16,
-                         uint4 *__restrict__ xp, uint32_t *__restrict__ slot, uint32_t pairs, uint32_t topk,
+                         uint4 *xp, uint32_t *slot, uint32_t pairs, uint32_t topk,
                          uint32_t d8, uint32_t ebound, uint4 *const *xp_peers, uint32_t experts_per_rank,
-                         uint32_t ppb, uint32_t *__restrict__ src_row, uint32_t *const *src_row_peers,
+                         uint32_t ppb, uint32_t *src_row, uint32_t *const *src_row_peers,
                          uint32_t src_base, uint2 *const *ret_peers, const float *wt) {
     moe_pdl_begin();
     // ppb = pairs per block (<= SC_MAX_PAIRS): 64 in the stand-alone scatter, 8*topk behind the fused router.

@@ -1,7 +1,7 @@
-"""Kernels that may be started while the one before them still runs (moe_run, moe_common.cuh) read what that one writes.
-`__ldg` and parameters declared `const T *__restrict__` promise data that is constant for the kernel's lifetime, which a
-compiler may use to move such a load in front of the wait; these kernels therefore use plain loads.  A property of the
-source text, checked as one."""
+"""Kernels that may be started while the one before them still runs (moe_run, moe_common.cuh) read what that one writes
+and write what it reads.  `__ldg` promises data that is constant for the kernel's lifetime and `__restrict__` that nothing
+else touches the object, so a compiler may move such accesses in front of the wait; these kernels therefore use plain loads
+and plain pointers.  A property of the source text, checked as one."""
 import glob
 import os
 import re
@@ -41,7 +41,7 @@ def test_every_early_kernel_is_found():
 def test_early_kernel_waits_and_loads_plainly(name):
     source, params, body = KERNELS[name]
     assert "moe_pdl_begin();" in body
-    assert not re.search(r"const\s+[\w ]+\*(\s*const\s*\*)?\s*__restrict__", params) and not re.search(r"\*const \*__restrict__", params)
+    assert "__restrict__" not in params
     helpers = [] if source in ("moe_ep.cu", "moe_kd.cu") else [SOURCES[source]]   # those two also hold kernels of serial launches
     for text in [body, SOURCES["moe_common.cuh"], SOURCES["moe_tc.cuh"]] + helpers:
         assert "__ldg(" not in text and "global.nc" not in text
