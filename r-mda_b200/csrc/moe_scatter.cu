@@ -183,7 +183,13 @@ moe_scatter_place_kernel(const uint32_t *idx, const uint32_t *off, const uint32_
                     dst[i + 64u] = c2;
                     dst[i + 96u] = d2;
                 }
-                for (; i < d8; i += 32u) dst[i] = src[i];  // :30-32
+                if (i + 32u < d8) {
+                    const uint4 a = src[i], b = src[i + 32u];
+                    dst[i] = a;
+                    dst[i + 32u] = b;
+                    i += 64u;
+                }
+                if (i < d8) dst[i] = src[i];  // :30-32
             }
             __syncthreads();  // the tables are rewritten by the next group
         }

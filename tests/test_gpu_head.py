@@ -15,7 +15,8 @@ def _f16(rng, shape, std):
 
 
 @pytest.mark.parametrize("rows,groups,gsize,op", [(37, 4, 256, 0), (5, 1, 2048, 0), (64, 4, 200, 1), (1, 3, 7, 0),
-                                                   (3, 2, 2052, 0), (2, 1, 4096, 1), (2, 1, 4100, 0), (5, 3, 4, 0)])
+                                                   (3, 2, 2052, 0), (2, 1, 4096, 1), (2, 1, 4100, 0), (5, 3, 4, 0),
+                                                   (3, 1, 8192, 0), (2, 1, 8196, 1), (3, 1, 8190, 0)])
 def test_norm(ctx, oracle, rows, groups, gsize, op):
     rng = np.random.default_rng(rows + gsize)
     x = rng.standard_normal((rows, groups * gsize)).astype(np.float32) * 3.0
@@ -38,9 +39,14 @@ def test_hc_read_out_widths(ctx, oracle, rows, d, hc):
     _check_hc(ctx, oracle, 0, rows, d, hc)
 
 
+@pytest.mark.parametrize("rows,d,hc", [(1, 1, 1), (5, 190, 3), (7, 64, 5), (3, 33, 9)])
+def test_hc_injection_widths(ctx, oracle, rows, d, hc):
+    _check_hc(ctx, oracle, 1, rows, d, hc)
+
+
 def _check_hc(ctx, oracle, op, rows, d, hc):
     rng = np.random.default_rng(op)
-    stride, off = 24, 17
+    stride, off = 32, 17
     if op == 0:
         a, b = rng.standard_normal((rows, hc * d)).astype(np.float32), rng.standard_normal((rows, hc * d)).astype(np.float32)
         h0 = np.full((rows, d), np.nan, np.float32)
