@@ -75,6 +75,8 @@ typedef struct moe_cuda_ctx moe_cuda_ctx_t;
 
 /* mda_vkc_init (src/vkc.c:95-161): bind one device and one in-order queue.
  * stream = an existing cudaStream_t to enqueue on, or NULL to create one.
+ * The context holds a work area of 512 KiB per SM (74 MiB) until it is
+ * destroyed; without memory for it the calls that use it do with less.
  * Returns NULL only if the context object itself cannot be made; otherwise
  * check moe_cuda_status(). */
 moe_cuda_ctx_t *moe_cuda_create(int device, void *stream);
@@ -191,7 +193,8 @@ void moe_cuda_norm(moe_cuda_ctx_t *c, const float *x, const float *w, float *y, 
 void moe_cuda_hc(moe_cuda_ctx_t *c, const float *a, const float *b, float *h, struct mda_pc_qwen_hc_t pc);
 /* mda_qwen_mm (src/qwen.c:541-570; shader/matmul_f16_wide.comp and the small-tile
  * kernel it alternates with): dense fp16 x fp16 -> fp32 product on the tcgen05
- * kernel of the grouped products.  n % 128 == 0, k % 8 == 0; any rows >= 1. */
+ * kernel of the grouped products.  n % 128 == 0, k % 8 == 0; any rows >= 1.
+ * Allocates nothing: the partial sums of a split K lie in the context's work area. */
 void moe_cuda_dense(moe_cuda_ctx_t *c, const void *A16, const void *W, float *C, const uint32_t *amax,
                     struct moe_pc_dense_t pc);
 

@@ -16,7 +16,10 @@
 #define MOE_TILE 128u         // MDA_QWEN_TILE, src/qwen.h:14
 
 // Scratch areas inside the context (grown on demand, never shrunk).
-enum { MOE_SCR_SCATTER = 0, MOE_SCR_LAYER = 1, MOE_SCR_STAGE = 2, MOE_SCR_EP = 3, MOE_SCR_KD = 4, MOE_SCR_COUNT = 5 };
+enum { MOE_SCR_SCATTER = 0, MOE_SCR_LAYER = 1, MOE_SCR_EP = 2, MOE_SCR_KD = 3, MOE_SCR_COUNT = 4 };
+// The context's fixed work area, made with the context and kept to its end: a call that uses it allocates nothing, and a
+// captured graph's pointers into it stay good.  Per SM two tiles of 256 x 256 fp32 sums, 74 MiB on 148 SMs.
+#define MOE_WORK_PER_SM ((size_t)2 * 256 * 256 * 4)
 
 // Tensor maps already made, by what they describe: a hash picks a set of MOE_TMAP_WAYS entries, a full set gives up its
 // entries in turn.  512 entries hold the weights of a 48-layer stack (3 per layer) beside everything else of a context;
@@ -56,6 +59,8 @@ struct moe_cuda_ctx {
     uint32_t *dev_status_dev;
     void *scratch[MOE_SCR_COUNT];
     size_t scratch_bytes[MOE_SCR_COUNT];
+    void *work;         // or NULL with work_bytes 0: no memory for it, callers do without
+    size_t work_bytes;
     moe_tmap_entry tmaps[MOE_TMAP_SETS][MOE_TMAP_WAYS];
     moe_xmap_entry xmaps[MOE_XMAP_SETS][MOE_TMAP_WAYS];
     uint8_t next_tmap[MOE_TMAP_SETS], next_xmap[MOE_XMAP_SETS];

@@ -47,17 +47,19 @@ extern "C" moe_cuda_ctx_t *moe_cuda_create(int device, void *stream) {
         moe_fail(c, MOE_ERR_CUDA, "no usable CUDA device %d: %s", device, cudaGetErrorString(e));
         return c;
     }
-    cudaDeviceProp prop;
-    e = cudaGetDeviceProperties(&prop, device);
+    // attributes one by one: cudaGetDeviceProperties takes 2.7 ms, more than all else here
+    int major = 0, minor = 0;
+    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) {
-        moe_fail(c, MOE_ERR_CUDA, "device properties: %s", cudaGetErrorString(e));
+        moe_fail(c, MOE_ERR_CUDA, "device attributes: %s", cudaGetErrorString(e));
         return c;
     }
-    if (prop.major != 10) {  // the kernels are built for sm_100a only (cf. src/vkc.c:49-64 feature checks)
-        moe_fail(c, MOE_ERR_UNSUPPORTED, "device %d is sm_%d%d, need sm_100", device, prop.major, prop.minor);
+    if (major != 10) {  // the kernels are built for sm_100a only (cf. src/vkc.c:49-64 feature checks)
+        moe_fail(c, MOE_ERR_UNSUPPORTED, "device %d is sm_%d%d, need sm_100", device, major, minor);
         return c;
     }
-    c->sm_count = prop.multiProcessorCount;
     if (stream != NULL) {
         c->stream = (cudaStream_t)stream;
     } else {
@@ -77,6 +79,12 @@ extern "C" moe_cuda_ctx_t *moe_cuda_create(int device, void *stream) {
         moe_fail(c, MOE_ERR_CUDA, "status word: %s", cudaGetErrorString(e));
         return c;
     }
+    c->work_bytes = (size_t)c->sm_count * MOE_WORK_PER_SM;
+    if (cudaMalloc(&c->work, c->work_bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->work = NULL;
+        c->work_bytes = 0;
+    }
     cudaDriverEntryPointQueryResult q;
     e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &c->encode_tiled, cudaEnableDefault, &q);
     if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || c->encode_tiled == NULL) {
@@ -93,6 +101,7 @@ extern "C" void moe_cuda_destroy(moe_cuda_ctx_t *c) {
     for (int i = 0; i < MOE_SCR_COUNT; i += 1) {
         if (c->scratch[i] != NULL) cudaFree(c->scratch[i]);
     }
+    if (c->work != NULL) cudaFree(c->work);
     if (c->ev_made) {
         for (int i = 0; i <= MOE_PROF_STAGES; i += 1) cudaEventDestroy(c->ev[i]);
     }

@@ -69,7 +69,8 @@ struct WsArgs {
     uint64_t wait_ns;
     // dense form (MM_DENSE): no chunk list, rows are cut into chunks of `per` (a multiple of 16)
     uint32_t rows, per;
-    uint32_t splits, ksplit;   // K split `splits` ways, ksplit K steps each; split p of C starts at C + p * rows * ldc
+    uint32_t splits, ksplit;   // K split `splits` ways, ksplit K steps each; the first one's sums go to C,
+    float *part;               // split p's to part + (p - 1) * rows * ldc
     const uint32_t *tiles;     // or NULL: expert of each 128-row tile, >= experts: the tile is skipped (per divides 128)
     uint32_t experts;
     const uint32_t *amax;      // scale slots (power of two) of both operands
@@ -448,7 +449,8 @@ moe_mm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 const uint32_t cfeat = (it.ft * PAIR + rank) * 128u + q * 32u + lane;
                 // dense form: the last pair may reach beyond n (n is a multiple of 128, not of 256)
                 const uint32_t nvalid = MODE == MM_DENSE && cfeat >= a.n ? 0u : it.nvalid;
-                float *C = reinterpret_cast<float *>(a.C) + (MODE == MM_DENSE ? (size_t)it.split * a.rows * a.ldc : 0u);
+                float *C = reinterpret_cast<float *>(a.C);
+                if (MODE == MM_DENSE && it.split != 0u) C = a.part + (size_t)(it.split - 1u) * a.rows * a.ldc;
 #pragma unroll 1
                 for (uint32_t cch = 0; cch < nch; cch += 1) {
                     uint32_t v[32];
@@ -498,15 +500,15 @@ moe_chunk_kernel(const uint32_t *__restrict__ count, const uint32_t *__restrict_
     moe_chunk_body(count, off, experts, chunks, n_chunks, max_chunks);
 }
 
-// C = the sum of the partial products of a split K, in split order.  n and with it every row is a multiple of four.
+// C += the partial products of the other splits of K, in split order.  n and with it every row is a multiple of four.
 __global__ void __launch_bounds__(256)
 moe_ksum_kernel(const float4 *part, float4 *C, uint32_t total4, uint32_t splits) {
     moe_pdl_begin();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= total4) return;
-    float4 acc = __ldcg(part + i);
+    float4 acc = C[i];
     for (uint32_t p = 1; p < splits; p += 1) {
-        const float4 v = __ldcg(part + (size_t)p * total4 + i);
+        const float4 v = __ldcg(part + (size_t)(p - 1u) * total4 + i);
         acc.x += v.x;
         acc.y += v.y;
         acc.z += v.z;
@@ -598,9 +600,10 @@ namespace {
 // Rows per item and K splits of the dense form: the pair with the least estimated time.  Unit: 128 bytes loaded into
 // an SM (1.8 ns at the 70 B/ns that an SM gets from L2).  A K step brings 128 weight rows and half of the item's token
 // rows of 128 bytes; an epilogue stores 512 bytes per token and is hidden but for the last one; a split costs a second
-// launch (4 us) and its partial sums a write and a read through L2 (5 TB/s).
+// launch (4 us) and its partial sums a write and a read through L2 (5 TB/s).  Splits whose sums beside C do not fit the
+// context's work area are not taken: nothing is allocated here.  The most that any shape tried asks for is 69 MiB.
 // 3001 x 384, K 8192: 34 us as 3 splits against 64 us whole on the token-major kernel; 384 x 384: 16 against 64 us.
-void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t kblocks, uint32_t clusters, bool tiled) {
+void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t kblocks, uint32_t clusters, bool tiled, size_t work_bytes) {
     const uint32_t nch0 = (rows + MAX_TOK - 1u) / MAX_TOK;
     uint64_t best = ~0ull;
     for (uint32_t i = 0; i < (tiled ? 3u : 4u); i += 1) {
@@ -613,11 +616,12 @@ void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t k
             const uint64_t waves = (items * s + clusters - 1u) / clusters;
             uint64_t t = waves * ks * (128u + per / 2u) + per * 4u;
             if (s > 1) t += 2200u + (uint64_t)s * rows * n * 8u / 9000u;
-            if (t < best) {
+            const uint32_t splits = (kblocks + ks - 1u) / ks;  // no empty split
+            if (t < best && (uint64_t)(splits - 1u) * rows * n * 4u <= work_bytes) {
                 best = t;
                 a.per = per;
                 a.ksplit = ks;
-                a.splits = (kblocks + ks - 1u) / ks;  // no empty split
+                a.splits = splits;
             }
             if (items * s >= 4u * (uint64_t)clusters) break;  // the last wave no longer matters
         }
@@ -627,8 +631,8 @@ void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t k
 
 // Dense product on the same kernel, pairs of CTAs only: C[rows x n] = X[rows x k] * W[e][n x k]^T / scales, where e is 0
 // or, with `tiles`, the expert of the 128-row tile.
-//   tiles == NULL: chunks of up to 256 rows; K may be split, the fp32 partial sums are then added in split order by a
-//     second kernel.
+//   tiles == NULL: chunks of up to 256 rows; K may be split, the fp32 partial sums (the first split's in C, the others' in
+//     the context's work area) are then added in split order by a second kernel.
 //   tiles != NULL: chunks of 128, 64 or 32 rows, K whole, no scratch.
 void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C, const uint32_t *amax, const uint32_t *tiles,
                          uint32_t rows, uint32_t n, uint32_t k, uint32_t sa, uint32_t sb, uint32_t experts_in_W) {
@@ -643,12 +647,9 @@ void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C
     if (!moe_tmap_2d_f16(c, &tmW, W, (uint64_t)experts_in_W * n, k, 128) || !moe_tmap_tokens_f16(c, &tmX, X, rows, k)) return;
     const uint32_t clusters = (uint32_t)c->sm_count / 2u, ft = (n + 255u) / 256u, kblocks = (k + BK - 1u) / BK;
     WsArgs a = {};
-    ws_dense_plan(a, rows, n, ft, kblocks, clusters, tiles != NULL);
+    ws_dense_plan(a, rows, n, ft, kblocks, clusters, tiles != NULL, c->work_bytes);
     a.C = C;
-    if (a.splits > 1) {
-        a.C = moe_scratch(c, MOE_SCR_STAGE, (size_t)a.splits * rows * n * 4);
-        if (a.C == NULL) return;
-    }
+    a.part = (float *)c->work;
     a.n = n;
     a.k = k;
     a.ldc = n;
@@ -665,7 +666,7 @@ void moe_launch_mm_dense(moe_cuda_ctx *c, const void *X, const void *W, float *C
     ws_launch<MM_DENSE, 2>(c, tmW, tmX, a, (uint32_t)(total < clusters ? total : clusters) * 2u);
     if (a.splits > 1 && MOE_LIVE(c)) {
         const uint32_t total4 = rows * (n / 4u);
-        moe_run(c, moe_ksum_kernel, (total4 + 255u) / 256u, 256, 0, (const float4 *)a.C, (float4 *)C, total4, a.splits);
+        moe_run(c, moe_ksum_kernel, (total4 + 255u) / 256u, 256, 0, (const float4 *)a.part, (float4 *)C, total4, a.splits);
         MOE_LAUNCHED(c);
     }
 }

@@ -99,6 +99,59 @@ def test_dense(ctx, oracle, rows, n, k, slot):
     assert np.all(np.abs(got[:rows] - ref) <= 1e-5 * np.abs(ref) + 1e-5 * np.abs(ref).max())   # same products, fp32 sums in another order
 
 
+def _dense_case(rng, rows, n, k):
+    a16, w16 = _f16(rng, (rows, k), 1.0), _f16(rng, (n, k), 0.05)
+    return a16, w16, a16.view(np.float16).astype(np.float32) @ w16.view(np.float16).astype(np.float32).T
+
+
+def test_dense_allocates_nothing(mc):
+    """Not the first call of a context, not a larger one: products with a split K live on the work area that is made with
+    the context.  An allocation would be refused here, and would show in the device's free memory."""
+    import torch
+    rng = np.random.default_rng(2)
+    with mc.Ctx(0) as c:
+        c.check()
+        cases = [(a, w, ref, c.upload(a), c.upload(w), c.alloc(ref.nbytes))
+                 for a, w, ref in (_dense_case(rng, rows, 384, 8192) for rows in (16, 384, 3001))]
+        c.flush()
+        free0, _ = torch.cuda.mem_get_info(0)
+        mc.lib().moe_cuda_fail_alloc_after(c.p, 1)
+        for a, w, ref, d_a, d_w, d_c in cases:
+            c.dense(d_a, d_w, d_c, None, len(a), 384, 8192)
+        c.flush()
+        assert torch.cuda.mem_get_info(0)[0] == free0
+        mc.lib().moe_cuda_fail_alloc_after(c.p, 0)
+        for a, w, ref, d_a, d_w, d_c in cases:
+            got = d_c.read(np.float32, ref.shape)
+            assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()   # fp32 sums of 8192 products in two orders
+
+
+def test_captured_dense_outlives_larger_calls(mc):
+    """A graph captured around a product with a split K still gives its result after larger products on the context."""
+    import torch
+    rng = np.random.default_rng(3)
+    stream = torch.cuda.Stream()
+    with mc.Ctx(0, stream.cuda_stream) as c:
+        c.check()
+        a, w, ref = _dense_case(rng, 64, 384, 8192)
+        la, lw, lref = _dense_case(rng, 3001, 384, 8192)
+        d_a, d_w, d_c, d_la, d_lw, d_lc = (c.upload(a), c.upload(w), c.alloc(ref.nbytes), c.upload(la), c.upload(lw), c.alloc(lref.nbytes))
+        c.dense(d_a, d_w, d_c, None, 64, 384, 8192)   # kernels loaded before the capture
+        c.flush()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            c.dense(d_a, d_w, d_c, None, 64, 384, 8192)
+        c.check()
+        c.dense(d_la, d_lw, d_lc, None, 3001, 384, 8192)
+        d_c.fill(0x7fc00000)
+        with torch.cuda.stream(stream):
+            g.replay()
+        c.flush()
+        assert np.abs(d_c.read(np.float32, ref.shape) - ref).max() <= 1e-5 * np.abs(ref).max()
+        assert np.abs(d_lc.read(np.float32, lref.shape) - lref).max() <= 1e-5 * np.abs(lref).max()
+        del g
+
+
 class Mix(C.Structure):
     _fields_ = ([("c", C.c_void_p)] + [(n, C.c_uint32) for n in ("d", "hc", "hc_rank", "hc_pad", "rows", "vocab")]
                 + [(n, C.c_void_p) for n in ("hn", "a16", "t", "u", "up", "x", "logits", "amax")] + [("n_slots", C.c_uint32)])
