@@ -210,7 +210,8 @@ void moe_cuda_bf16_to_f16(moe_cuda_ctx_t *c, void *w, struct mda_pc_qwen_bf16_t 
  * bytes of the token (little-endian in four words) and its length, 0 = no byte
  * string; cont [rows x 5]: the 16 bytes that follow the row's position and how
  * many of them count; outp [rows x 16 x 8] entries byte | fp16(p) << 16 -- per
- * depth the true byte's probability, then the seven most probable other bytes. */
+ * depth the true byte's probability, then the seven most probable other bytes.
+ * Scratch grows with the vocabulary only, not with the rows. */
 void moe_cuda_kd_bytes(moe_cuda_ctx_t *c, const float *logits, const uint32_t *toks, const uint32_t *cont,
                        uint32_t *outp, struct mda_pc_kd_bytes_t pc);
 

@@ -68,15 +68,14 @@ __device__ __forceinline__ uint32_t kd_pack_entry(uint32_t b, float p) {  // :70
     return b | ((uint32_t)__half_as_ushort(__float2half_rn(p)) << 16);
 }
 
-// One block per batch of rows: rows [b * batch, ...) in order of their continuation's first byte, so that the 32 rows of a
-// block of the sweep share few first bytes and most runs of the sweep end at a first byte only.
+// The block behind them: the rows of a batch in order of their continuation's first byte, so that the 32 rows of a block of the sweep
+// share few first bytes and most runs of the sweep end at a first byte only.
 #define KD_SORT_THREADS (KD_SORTED / 8u)
-__device__ __forceinline__ void kd_order_rows(uint32_t *s, const uint32_t *cont, uint32_t *row_map, uint32_t rows, uint32_t b, uint32_t batch) {
-    const uint32_t lo = b * batch, hi = min(lo + batch, rows);
+__device__ __forceinline__ void kd_order_rows(uint32_t *s, const uint32_t *cont, uint32_t *row_map, uint32_t rows) {
     for (uint32_t i = threadIdx.x; i < 256u; i += KD_SORT_THREADS) s[i] = 0u;
     __syncthreads();
 #pragma unroll 4
-    for (uint32_t r = lo + threadIdx.x; r < hi; r += KD_SORT_THREADS) atomicAdd(&s[cont[(size_t)r * 5u] & 0xffu], 1u);
+    for (uint32_t r = threadIdx.x; r < rows; r += KD_SORT_THREADS) atomicAdd(&s[cont[(size_t)r * 5u] & 0xffu], 1u);
     __syncthreads();
     if (threadIdx.x < 32u) {
         uint32_t n[8], sum = 0;
@@ -88,7 +87,7 @@ __device__ __forceinline__ void kd_order_rows(uint32_t *s, const uint32_t *cont,
             const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
             if (threadIdx.x >= o) incl += u;
         }
-        uint32_t at = lo + incl - sum;
+        uint32_t at = incl - sum;
 #pragma unroll
         for (uint32_t i = 0; i < 8; i += 1) {
             s[threadIdx.x * 8u + i] = at;
@@ -97,18 +96,17 @@ __device__ __forceinline__ void kd_order_rows(uint32_t *s, const uint32_t *cont,
     }
     __syncthreads();
 #pragma unroll 4
-    for (uint32_t r = lo + threadIdx.x; r < hi; r += KD_SORT_THREADS) row_map[atomicAdd(&s[cont[(size_t)r * 5u] & 0xffu], 1u)] = r;
+    for (uint32_t r = threadIdx.x; r < rows; r += KD_SORT_THREADS) row_map[atomicAdd(&s[cont[(size_t)r * 5u] & 0xffu], 1u)] = r;
 }
 
-// One block per chunk: bitonic sort of eight consecutive entries per thread.  Strides below 8 are register to register,
-// up to 128 by shuffle, so 52 of the 55 steps need no barrier (with one entry per thread: 13.5 us a call, now 5).
+// The first n_chunks blocks, one per chunk: bitonic sort of eight consecutive entries per thread.  Strides below 8 are
+// register to register, up to 128 by shuffle, so 52 of the 55 steps need no barrier (with one entry per thread: 13.5 us a call, now 5).
 __global__ void __launch_bounds__(KD_SORT_THREADS)
 moe_kd_sort_kernel(const uint32_t *__restrict__ toks, uint32_t *__restrict__ sorted, uint4 *__restrict__ bytes, uint32_t vocab,
-                   const uint32_t *__restrict__ cont, uint32_t *__restrict__ row_map, uint32_t rows, uint32_t batch) {
+                   const uint32_t *__restrict__ cont, uint32_t *__restrict__ row_map, uint32_t rows, uint32_t n_chunks) {
     __shared__ uint32_t s[KD_SORTED];
-    const uint32_t n_chunks = (vocab + KD_CHUNK - 1u) / KD_CHUNK;
     if (blockIdx.x >= n_chunks) {
-        kd_order_rows(s, cont, row_map, rows, blockIdx.x - n_chunks, batch);
+        kd_order_rows(s, cont, row_map, rows);
         return;
     }
     const uint32_t i0 = threadIdx.x * 8u, t0 = blockIdx.x * KD_CHUNK + i0;
@@ -559,51 +557,65 @@ moe_kd_rows_kernel(const float *__restrict__ logits, const uint4 *__restrict__ b
     }
 }
 
+// Rows in batches of `groups` groups of 32, the chunk list of each cut `splits` ways: two blocks per SM, and the rounds of
+// blocks (each a share of the chunks plus ~2 chunks' worth of set-up and write-out, a further batch ~4) take the least time.
+// The bins of a batch's blocks, at most max_blocks, lie in the work area: up to 2800 rows (of a vocabulary of 256,000; 4200
+// of 151,936) that decides nothing, beyond it more batches take the place of more blocks.
+static void kd_plan(uint32_t groups_all, uint32_t n_chunks, uint32_t slots, size_t max_blocks, uint32_t *groups, uint32_t *splits) {
+    const uint32_t least = (groups_all + slots - 1u) / slots;
+    uint64_t best = ~0ull;
+    for (uint32_t n = least; n < least + 8u && n <= groups_all; n += 1) {
+        const uint32_t g = (groups_all + n - 1u) / n;
+        for (uint32_t s = 1; s <= n_chunks && s <= KD_MAX_SPLITS && (size_t)g * s <= max_blocks; s += 1) {
+            const uint64_t cost = (uint64_t)n * (((g * s + slots - 1u) / slots) * (uint64_t)((n_chunks + s - 1u) / s + 2u) + (n > 1u ? 4u : 0u));
+            if (cost < best) {
+                best = cost;
+                *groups = g;
+                *splits = s;
+            }
+        }
+    }
+}
+
 extern "C" void moe_cuda_kd_bytes(moe_cuda_ctx_t *c, const float *logits, const uint32_t *toks, const uint32_t *cont,
                                   uint32_t *outp, struct mda_pc_kd_bytes_t pc) {
     if (!MOE_LIVE(c)) return;
     MOE_REQUIRE(c, logits != NULL && toks != NULL && cont != NULL && outp != NULL, "kd_bytes: null buffer");
     MOE_REQUIRE(c, pc.vocab >= 1, "kd_bytes: empty vocabulary");
     if (pc.rows == 0) return;
-    const uint32_t n_chunks = (pc.vocab + KD_CHUNK - 1u) / KD_CHUNK;
-    // Two blocks per SM: rows in batches of at most that many groups, the chunk list cut so that the rounds of blocks
-    // (each a share of the chunks plus ~2 chunks' worth of set-up and write-out) take the least time.
-    const uint32_t slots = 2u * (uint32_t)c->sm_count;
-    const uint32_t groups_all = (pc.rows + KD_ROWS - 1u) / KD_ROWS, groups_max = groups_all < slots ? groups_all : slots;
-    uint32_t splits = 1;
-    uint64_t best = ~0ull;
-    for (uint32_t s = 1; s <= n_chunks && s <= KD_MAX_SPLITS; s += 1) {
-        const uint64_t cost = (uint64_t)((groups_max * s + slots - 1u) / slots) * ((n_chunks + s - 1u) / s + 2u);
-        if (cost < best) {
-            best = cost;
-            splits = s;
-        }
-    }
-    const size_t blocks_max = (size_t)groups_max * splits, tokens = (size_t)n_chunks * KD_CHUNK;
-    const size_t bins_bytes = blocks_max * KD_ROWS * KD_BINS * sizeof(float);
-    uint8_t *scr = (uint8_t *)moe_scratch(c, MOE_SCR_KD, tokens * (sizeof(uint4) + sizeof(uint32_t)) + bins_bytes +
-                                                                blocks_max * KD_ROWS * sizeof(float2) + (size_t)pc.rows * sizeof(uint32_t));
+    // Scratch grows with the vocabulary only; what depends on the rows lies in the context's work area (without one, in
+    // scratch for one round of blocks).
+    const uint32_t n_chunks = (pc.vocab + KD_CHUNK - 1u) / KD_CHUNK, slots = 2u * (uint32_t)c->sm_count;
+    const size_t tokens = (size_t)n_chunks * KD_CHUNK, block_bytes = KD_ROWS * (KD_BINS * sizeof(float) + sizeof(float2));
+    const size_t max_blocks = c->work != NULL ? c->work_bytes / block_bytes : slots;
+    uint8_t *scr = (uint8_t *)moe_scratch(c, MOE_SCR_KD, tokens * (sizeof(uint4) + sizeof(uint32_t)) + (size_t)slots * KD_ROWS * sizeof(uint32_t) +
+                                                             (c->work != NULL ? 0 : max_blocks * block_bytes));
     if (scr == NULL) return;
+    uint32_t groups = 1, splits = 1;
+    kd_plan((pc.rows + KD_ROWS - 1u) / KD_ROWS, n_chunks, slots, max_blocks, &groups, &splits);
     uint4 *bytes = (uint4 *)scr;
-    float *bins = (float *)(bytes + tokens);
-    float2 *refs = (float2 *)(bins + bins_bytes / sizeof(float));
-    uint32_t *sorted = (uint32_t *)(refs + blocks_max * KD_ROWS);
-    uint32_t *row_map = sorted + tokens;
+    uint32_t *sorted = (uint32_t *)(bytes + tokens);
+    uint32_t *row_map = sorted + tokens;  // of a batch
+    float *bins = (float *)(c->work != NULL ? c->work : (void *)(row_map + slots * KD_ROWS));
+    float2 *refs = (float2 *)(bins + (size_t)groups * splits * KD_ROWS * KD_BINS);
     const bool vec = pc.vocab % 4u == 0 && ((uintptr_t)logits & 15) == 0;
     if (!c->kd_attr_set) {
         MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_kd_mass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(kd_mass_smem)));
         MOE_CUDA_TRY(c, cudaFuncSetAttribute(moe_kd_mass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(kd_mass_smem)));
         c->kd_attr_set = true;
     }
-    const uint32_t batch = groups_max * KD_ROWS, batches = (pc.rows + batch - 1u) / batch;
-    moe_kd_sort_kernel<<<n_chunks + batches, KD_SORT_THREADS, 0, c->stream>>>(toks, sorted, bytes, pc.vocab, cont, row_map, pc.rows, batch);
-    MOE_LAUNCHED(c);
-    for (uint32_t row0 = 0; row0 < pc.rows; row0 += batch) {  // row_map holds rows of the whole call
-        const uint32_t rows = pc.rows - row0 < batch ? pc.rows - row0 : batch, groups = (rows + KD_ROWS - 1u) / KD_ROWS;
-        if (vec) moe_kd_mass_kernel<true><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, refs, pc.vocab, rows, splits);
-        else moe_kd_mass_kernel<false><<<groups * splits, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(logits, sorted, cont, row_map + row0, bins, refs, pc.vocab, rows, splits);
+    const uint32_t batch = groups * KD_ROWS;
+    for (uint32_t row0 = 0; row0 < pc.rows; row0 += batch) {
+        const uint32_t rows = pc.rows - row0 < batch ? pc.rows - row0 : batch, blocks = (rows + KD_ROWS - 1u) / KD_ROWS * splits;
+        const uint32_t sort = row0 == 0 ? n_chunks : 0u;  // the chunks serve all batches
+        const float *lg = logits + (size_t)row0 * pc.vocab;
+        const uint32_t *ct = cont + (size_t)row0 * 5u;
+        moe_kd_sort_kernel<<<sort + 1u, KD_SORT_THREADS, 0, c->stream>>>(toks, sorted, bytes, pc.vocab, ct, row_map, rows, sort);
         MOE_LAUNCHED(c);
-        moe_kd_rows_kernel<<<rows, KD_RTHREADS, 0, c->stream>>>(logits, bytes, sorted, cont, row_map + row0, bins, refs, outp, pc.vocab, splits);
+        if (vec) moe_kd_mass_kernel<true><<<blocks, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(lg, sorted, ct, row_map, bins, refs, pc.vocab, rows, splits);
+        else moe_kd_mass_kernel<false><<<blocks, KD_THREADS, sizeof(kd_mass_smem), c->stream>>>(lg, sorted, ct, row_map, bins, refs, pc.vocab, rows, splits);
+        MOE_LAUNCHED(c);
+        moe_kd_rows_kernel<<<rows, KD_RTHREADS, 0, c->stream>>>(lg, bytes, sorted, ct, row_map, bins, refs, outp + (size_t)row0 * KD_D * KD_K, pc.vocab, splits);
         MOE_LAUNCHED(c);
     }
 }

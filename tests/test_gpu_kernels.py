@@ -361,6 +361,22 @@ def test_kd_bytes_special_logits(ctx, oracle, rows, vocab):
     assert ((got & 0xffff) != (ref & 0xffff)).mean() < 0.01
 
 
+def test_kd_bytes_scratch_depends_on_the_vocabulary_only(ctx, mc, oracle):
+    """After one call with a vocabulary no call with it allocates, whatever its rows."""
+    from tests.test_oracle import kd_inputs
+    logits, toks, cont = kd_inputs(51, 512, 20000)
+    d_lg, d_toks, d_cont, d_out = ctx.upload(logits), ctx.upload(toks), ctx.upload(cont), ctx.alloc(512 * 16 * 8 * 4)
+    ctx.kd_bytes(d_lg, d_toks, d_cont, d_out, 8, 20000)
+    mc.lib().moe_cuda_fail_alloc_after(ctx.p, 1)
+    ctx.kd_bytes(d_lg, d_toks, d_cont, d_out, 512, 20000)
+    ctx.flush()
+    mc.lib().moe_cuda_fail_alloc_after(ctx.p, 0)
+    got, ref = d_out.read(np.uint32, (512, 16, 8)), oracle.kd_bytes(logits, toks, cont)
+    pg = (got >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    pr = (ref >> 16).astype(np.uint16).view(np.float16).astype(np.float64)
+    assert np.all(np.abs(pg - pr) <= 1.5e-3 * pr + 1e-7)
+
+
 def test_fill_and_copy(ctx):
     b = ctx.alloc(4 * 1003)
     b.fill(0x12345678)
