@@ -152,11 +152,25 @@ def _f16(rng, shape, std):
 @pytest.mark.parametrize("m,n,k,E,sa", [
     (128, 128, 64, 1, False), (128, 256, 64, 1, False), (256, 384, 128, 3, False), (512, 1024, 256, 4, True),
     (384, 640, 96, 2, False), (1280, 256, 2048, 8, False), (256, 2048, 768, 5, True), (128, 128, 8, 1, False),
-    (4736, 256, 128, 3, True), (4864, 256, 128, 3, True), (2048, 384, 200, 1, False),  # either side of the idle-SM rule
+    (4736, 256, 128, 3, True), (4864, 256, 128, 3, True), (2048, 384, 200, 1, False),
 ])
 def test_mm(ctx, oracle, mc, m, n, k, E, sa):
     """moe_cuda_mm against the oracle's product: same tile schedule, skipped tiles untouched,
     slot scale applied.  Covers one K block, ragged K (96, 8), the 128-column tail, many experts."""
+    _check_mm(ctx, oracle, mc, m, n, k, E, sa)
+
+
+@pytest.mark.parametrize("n,k,E,sa", [(256, 128, 3, True), (384, 200, 3, False), (128, 72, 2, True)])
+@pytest.mark.parametrize("past", [0, 1])
+def test_mm_either_side_of_the_idle_sm_rule(ctx, oracle, mc, past, n, k, E, sa):
+    """moe_cuda_mm goes to the weight-stationary kernel while 128 x 256 tiles are at most half as many as SMs: the most row
+    tiles of that side, and one more.  Skipped tiles, a scale slot, a 128-column tail and a ragged K on both."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    _check_mm(ctx, oracle, mc, 128 * (sms // 2 // ((n + 255) // 256) + past), n, k, E, sa)
+
+
+def _check_mm(ctx, oracle, mc, m, n, k, E, sa):
     rng = np.random.default_rng(m + n + k)
     A = _f16(rng, (m, k), 1.0)
     B = _f16(rng, (E, n, k), 0.05)
@@ -302,10 +316,35 @@ def test_kd_bytes(ctx, oracle):
 
 
 @pytest.mark.parametrize("rows,vocab,alphabet,lift", [
-    (1, 1, 4, 0.0), (3, 1023, 4, 0.0), (33, 1025, 2, 0.0), (32, 4096, 1, 0.0), (65, 2049, 26, 130.0), (7, 5000, 250, -130.0)])
+    (1, 1, 4, 0.0), (3, 1023, 4, 0.0), (33, 1025, 2, 0.0), (32, 4096, 1, 0.0), (65, 2049, 26, 130.0), (7, 5000, 250, -130.0),
+    (3, 767, 4, 0.0), (31, 768, 4, 0.0), (33, 769, 4, 0.0), (64, 1536, 3, 130.0), (2, 1537, 4, 0.0), (3, 394001, 4, 0.0)])
 def test_kd_bytes_edges(ctx, oracle, rows, vocab, alphabet, lift):
-    """Edges of the 1024-token chunks and 32-row groups; all tokens behind the same bytes (alphabet 1); a row maximum
-    that a later chunk exceeds by more than the reference may lag (lift added to the last 600 logits)."""
+    """Edges of the 768-token chunks and 32-row groups; all tokens behind the same bytes (alphabet 1); splits of the chunk
+    list whose maxima are far apart (lift added to the last 600 logits); more than the 512 chunks that the kernel of the
+    rows looks at together.  Each block of the sweep has one chunk here, two in the last case."""
+    _check_kd(ctx, oracle, rows, vocab, alphabet, lambda lg, rng: _lift_last(lg, lift))
+
+
+def _lift_last(logits, lift):
+    logits[:, -600:] += np.float32(lift)
+
+
+@pytest.mark.parametrize("rows,vocab,shift", [(1280, 20000, 0), (1280, 20000, 1), (9500, 3100, 0)])
+def test_kd_bytes_several_chunks_per_block(ctx, oracle, rows, vocab, shift):
+    """A block of the sweep goes over four or five chunks (148 SMs): 40 row groups in 7 splits of 27 chunks; 9500 rows in two
+    batches of 149 and 148 groups, the 5 chunks whole.  Rows whose chunks rise by more than the reference may lag, once and
+    at every chunk, that fall, and that start or end in masked chunks.  `shift` floats off 16 bytes."""
+    def spoil(lg, rng):
+        step = np.repeat(np.arange(-(-vocab // 768)), 768)[:vocab].astype(np.float32)
+        lg[1::6] += 45.0 * step            # a new reference at every chunk
+        lg[2::6] -= 45.0 * step
+        lg[3::6, :2000] = -np.inf
+        lg[4::6, -2000:] = -np.inf
+        lg[5::6, 1600:1700] += 41.0        # just beyond the lag, once
+    _check_kd(ctx, oracle, rows, vocab, 4, spoil, shift)
+
+
+def _check_kd(ctx, oracle, rows, vocab, alphabet, spoil, shift=0):
     rng = np.random.default_rng(vocab)
     length = rng.integers(0, 17, vocab)
     tb = rng.integers(3, 3 + alphabet, (vocab, 16)).astype(np.uint8)
@@ -315,9 +354,10 @@ def test_kd_bytes_edges(ctx, oracle, rows, vocab, alphabet, lift):
     cont[:, :4] = rng.integers(3, 3 + alphabet, (rows, 16)).astype(np.uint8).view(np.uint32).reshape(rows, 4)
     cont[:, 4] = [16, 1, 2, 3, 0, 40][:rows] if rows <= 6 else rng.integers(0, 18, rows)
     logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
-    logits[:, -600:] += np.float32(lift)
+    spoil(logits, rng)
     d_out = ctx.alloc(rows * 16 * 8 * 4).fill(0xdeadbeef)
-    ctx.kd_bytes(ctx.upload(logits), ctx.upload(toks), ctx.upload(cont), d_out, rows, vocab)
+    d_lg = ctx.upload(np.concatenate([np.full(shift, 1e9, np.float32), logits.ravel()]))
+    ctx.kd_bytes(d_lg.ptr + 4 * shift, ctx.upload(toks), ctx.upload(cont), d_out, rows, vocab)
     ctx.flush()
     got, ref = d_out.read(np.uint32, (rows, 16, 8)), oracle.kd_bytes(logits, toks, cont)
     pg = (got >> 16).astype(np.uint16).view(np.float16).astype(np.float64)

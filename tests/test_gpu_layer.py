@@ -162,17 +162,27 @@ def test_upstream_projection_on_gpu_then_layer(ctx, mc, synth, oracle):
 
 
 def test_many_tensor_maps_in_one_context(ctx, mc, synth, oracle):
-    """More operand buffers than a context keeps tensor maps for: the maps of a launch stay those of its own operands."""
+    """More operand buffers than a context keeps tensor maps for (512 of weights and token-major operands, 32 of
+    weight-stationary products' tokens): the maps of a launch stay those of its own operands, also of those that come again
+    after theirs was replaced.  Every operand has values of its own, so that a mixed-up map changes a result."""
     import dataclasses
     cfg = dataclasses.replace(synth.CONFIGS["c0"], T=200, name="c0-T200")
     inp = synth.layer_inputs(cfg, 5)
     ref = oracle.layer(inp.proj, inp.x16, inp.wgu, inp.wdown, cfg.K)
     first = run_layer(ctx, mc, cfg, inp)
     check(first, ref)
-    n = 700
-    a, w, out = ctx.zeros((n + 1) * 16 * 64), ctx.zeros(128 * 8 * 2), ctx.alloc(8 * 128 * 4)
-    for i in range(n):
-        ctx.dense(a.ptr + i * 16 * 64, w, out, None, 8, 128, 8)
+    n, rows, k, cols = 700, 8, 8, 128
+    rng = np.random.default_rng(6)
+    a16, w16 = (rng.standard_normal(sh).astype(np.float16) for sh in ((n, rows, k), (n, cols, k)))
+    a, w, out = ctx.upload(a16.view(np.uint16)), ctx.upload(w16.view(np.uint16)), ctx.alloc(n * rows * cols * 4)
+    want = np.einsum("irk,ick->irc", a16.astype(np.float64), w16.astype(np.float64))
+    for order in (range(n), range(n - 1, -1, -1)):
+        out.fill(0x7fc00000)
+        for i in order:
+            ctx.dense(a.ptr + i * rows * k * 2, w.ptr + i * cols * k * 2, out.ptr + i * rows * cols * 4, None, rows, cols, k)
+        ctx.flush()
+        got = out.read(np.float32, want.shape)
+        assert np.abs(got - want).max() <= 1e-6 * np.abs(want).max()   # eight products, summed in fp32
     small = dataclasses.replace(cfg, T=72, name="c0-T72")
     part = synth.layer_inputs(small, 5)
     check(run_layer(ctx, mc, small, part), oracle.layer(part.proj, part.x16, part.wgu, part.wdown, cfg.K))
