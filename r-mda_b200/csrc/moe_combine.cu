@@ -335,10 +335,10 @@ extern "C" void moe_cuda_swiglu(moe_cuda_ctx_t *c, const float *a, float *y, str
         const uint32_t total4 = (uint32_t)(total / 4), blocks = (total4 + 2u * EL_THREADS - 1u) / (2u * EL_THREADS);
         if (pc.op == 0u)
             moe_run(c, moe_swiglu4_kernel<0>, blocks, EL_THREADS, 0, (const float4 *)a, (float4 *)y, total4, pc.n / 4u,
-                                                                       pc.astride / 4u, pc.ao / 4u, pc.bo / 4u, pc.scale);
+                    pc.astride / 4u, pc.ao / 4u, pc.bo / 4u, pc.scale);
         else
             moe_run(c, moe_swiglu4_kernel<1>, blocks, EL_THREADS, 0, (const float4 *)a, (float4 *)y, total4, pc.n / 4u,
-                                                                       pc.astride / 4u, pc.ao / 4u, 0, pc.scale);
+                    pc.astride / 4u, pc.ao / 4u, 0, pc.scale);
         MOE_LAUNCHED(c);
         return;
     }

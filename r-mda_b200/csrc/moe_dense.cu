@@ -182,8 +182,8 @@ extern "C" void moe_cuda_hc(moe_cuda_ctx_t *c, const float *a, const float *b, f
     // the teacher's four streams; other counts and ragged or unaligned rows take the general form below
     if (pc.op == 0u && pc.hc == 4u && pc.d % 4u == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)h) % 16 == 0 && n / 4 < (1ull << 31)) {
         const uint32_t total4 = (uint32_t)(n / 4);
-        moe_run(c, moe_hc_read4_kernel<4>, (total4 + NR_THREADS - 1u) / NR_THREADS, NR_THREADS, 0, 
-            (const float4 *)a, (const float4 *)b, (float4 *)h, total4, pc.d / 4u);
+        moe_run(c, moe_hc_read4_kernel<4>, (total4 + NR_THREADS - 1u) / NR_THREADS, NR_THREADS, 0,
+                (const float4 *)a, (const float4 *)b, (float4 *)h, total4, pc.d / 4u);
         MOE_LAUNCHED(c);
         return;
     }

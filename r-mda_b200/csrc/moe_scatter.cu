@@ -144,12 +144,13 @@ moe_scatter_place_kernel(const uint32_t *idx, const uint32_t *off, const uint32_
                 // expert-parallel: the row goes straight into the owning GPU's buffer over NVLink
                 s_dst[threadIdx.x] = xp_peers != NULL ? xp_peers[e / experts_per_rank] : xp;
                 if (first) slot[p0 + threadIdx.x] = p;  // :27
-                // gather mode: record where the row comes from instead of copying it; the product fetches it
-                if (!first) {
-                } else if (src_row != NULL) src_row[p] = (p0 + threadIdx.x) / topk;
-                // expert-parallel gather mode: the record goes into the owning GPU's table; the row itself
-                // travels once per destination GPU (moe_ep_send_kernel) and sits at src_base + its local index
-                else if (src_row_peers != NULL) {
+                // gather modes have one block per group: `first` holds in them
+                if (src_row != NULL) {
+                    // record where the row comes from instead of copying it; the product fetches it
+                    src_row[p] = (p0 + threadIdx.x) / topk;
+                } else if (src_row_peers != NULL) {
+                    // expert-parallel: the record goes into the owning GPU's table; the row itself travels once per
+                    // destination GPU (moe_ep_send_kernel) and sits at src_base + its local index
                     const uint32_t g = e / experts_per_rank, row = src_base + (p0 + threadIdx.x) / topk;
                     src_row_peers[g][p] = row;
                     if (ret_peers != NULL) {
@@ -218,14 +219,14 @@ void moe_launch_scatter(moe_cuda_ctx *c, const uint32_t *idx, const uint32_t *of
     uint32_t nblocks = (pairs + SC_PAIRS - 1) / SC_PAIRS;
     uint32_t *hist = (uint32_t *)moe_scratch(c, MOE_SCR_SCATTER, (size_t)nblocks * ebound * sizeof(uint32_t));
     if (hist == NULL) return;
-    moe_run(c, moe_scatter_hist_kernel, nblocks, SC_PAIRS, ebound * sizeof(uint32_t), idx, hist, pairs, ebound,
-                                                                                         c->dev_status_dev);
+    moe_run(c, moe_scatter_hist_kernel, nblocks, SC_PAIRS, ebound * sizeof(uint32_t), idx, hist, pairs, ebound, c->dev_status_dev);
     MOE_LAUNCHED(c);
-    moe_run(c, moe_scatter_colscan_kernel, (ebound + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, fill, nblocks, ebound, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
+    moe_run(c, moe_scatter_colscan_kernel, (ebound + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, fill, nblocks, ebound,
+            nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
     MOE_LAUNCHED(c);
-    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, sc_copy_split(c, nblocks, SC_PAIRS)), SC_THREADS, 0, idx, off, hist, (const uint4 *)x16, (uint4 *)xp,
-                                                                    slot, pairs, topk, d8, ebound,
-                                                                    (uint4 *const *)xp_peers, experts_per_rank, SC_PAIRS, nullptr, nullptr, 0, nullptr, nullptr);
+    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, sc_copy_split(c, nblocks, SC_PAIRS)), SC_THREADS, 0, idx, off, hist,
+            (const uint4 *)x16, (uint4 *)xp, slot, pairs, topk, d8, ebound, (uint4 *const *)xp_peers, experts_per_rank, SC_PAIRS,
+            nullptr, nullptr, 0, nullptr, nullptr);
     MOE_LAUNCHED(c);
 }
 
@@ -246,9 +247,8 @@ void moe_launch_colscan_counts(moe_cuda_ctx *c, uint32_t *hist, uint32_t *count,
         }
         ticket = c->ticket;
     }
-    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, nullptr, nblocks, experts, count,
-                                                                                                 ticket, off, tiles, tile,
-                                                                                                 (uint4 *)chunks, n_chunks, max_chunks);
+    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, hist, nullptr, nblocks, experts,
+            count, ticket, off, tiles, tile, (uint4 *)chunks, n_chunks, max_chunks);
     MOE_LAUNCHED(c);
 }
 
@@ -270,10 +270,9 @@ void moe_launch_place(moe_cuda_ctx *c, const uint32_t *idx, const uint32_t *off,
     uint32_t nblocks = (rows + 7u) / 8u;
     // gather modes copy nothing
     const uint32_t split = src_row == NULL && src_row_peers == NULL ? sc_copy_split(c, nblocks, 8u * topk) : 1u;
-    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, split), SC_THREADS, 0, idx, off, hist, (const uint4 *)x16, (uint4 *)xp, slot,
-                                                                    rows * topk, topk, d8, experts,
-                                                                    (uint4 *const *)xp_peers, experts_per_rank, 8u * topk, src_row,
-                                                                    src_row_peers, src_base, ret_peers, wt);
+    moe_run(c, moe_scatter_place_kernel, dim3(nblocks, split), SC_THREADS, 0, idx, off, hist, (const uint4 *)x16, (uint4 *)xp,
+            slot, rows * topk, topk, d8, experts, (uint4 *const *)xp_peers, experts_per_rank, 8u * topk, src_row, src_row_peers,
+            src_base, ret_peers, wt);
     MOE_LAUNCHED(c);
 }
 
@@ -330,12 +329,14 @@ extern "C" void moe_cuda_scatter_noalloc(moe_cuda_ctx_t *c, const uint32_t *idx,
     if (pairs == 0) return;
     // The table keeps the previous call's contents; nothing has to start at zero
     // because the hist kernel writes every entry the later kernels read.
-    moe_run(c, moe_scatter_hist_kernel, (uint32_t)nblocks, SC_PAIRS, experts * sizeof(uint32_t), 
-        idx, table, (uint32_t)pairs, experts, c->dev_status_dev);
+    moe_run(c, moe_scatter_hist_kernel, (uint32_t)nblocks, SC_PAIRS, experts * sizeof(uint32_t), idx, table,
+            (uint32_t)pairs, experts, c->dev_status_dev);
     MOE_LAUNCHED(c);
-    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, table, fill, (uint32_t)nblocks, experts, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
+    moe_run(c, moe_scatter_colscan_kernel, (experts + CS_EXPERTS - 1u) / CS_EXPERTS, 1024, 0, table, fill,
+            (uint32_t)nblocks, experts, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0);
     MOE_LAUNCHED(c);
-    moe_run(c, moe_scatter_place_kernel, dim3((uint32_t)nblocks, sc_copy_split(c, (uint32_t)nblocks, SC_PAIRS)), SC_THREADS, 0, 
-        idx, off, table, (const uint4 *)x16, (uint4 *)xp, slot, (uint32_t)pairs, pc.topk, pc.d8, experts, nullptr, 0, SC_PAIRS, nullptr, nullptr, 0, nullptr, nullptr);
+    moe_run(c, moe_scatter_place_kernel, dim3((uint32_t)nblocks, sc_copy_split(c, (uint32_t)nblocks, SC_PAIRS)), SC_THREADS, 0,
+            idx, off, table, (const uint4 *)x16, (uint4 *)xp, slot, (uint32_t)pairs, pc.topk, pc.d8, experts, nullptr, 0,
+            SC_PAIRS, nullptr, nullptr, 0, nullptr, nullptr);
     MOE_LAUNCHED(c);
 }
