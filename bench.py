@@ -503,7 +503,9 @@ def run_kd(args, ctx, mc, stream, local):
     ctx.flush()
     sampler = ClockSampler(local)
     sampler.start()
+    launched = ctx.launches()
     ms = timed_steps(torch, stream, fn, args.steps)
+    launched = ctx.launches() - launched
     clocks = sampler.stop()
     ctx.check()
     parity = {"checked": False}
@@ -526,8 +528,8 @@ def run_kd(args, ctx, mc, stream, local):
            "n_gpus": 1, "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True,
            "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
            "config": {"workload": "kd: 1024 rows x 151936 logits, 16 depths x 8 entries out", "l2": "622 MB of logits per step, larger than L2"},
-           "gpu_launches": 2 * args.steps, "clocks": clocks, "parity": parity,
-           "roofline": {"bound": "hbm", "kernel": "moe_kd_bytes_kernel (+ moe_kd_sort_kernel once per call)", "achieved": gbs,
+           "gpu_launches": launched, "clocks": clocks, "parity": parity,
+           "roofline": {"bound": "hbm", "kernel": "moe_kd_sort_kernel + moe_kd_mass_kernel + moe_kd_rows_kernel", "achieved": gbs,
                         "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": gbs / pk["hbm_gbs"], "traffic": None,
                         "peak_source": pk["source"], "bytes_per_launch": nbytes, "ms_per_launch": ms}}
     ctx.close()
