@@ -602,7 +602,8 @@ namespace {
 // rows of 128 bytes; an epilogue stores 512 bytes per token and is hidden but for the last one; a split costs a second
 // launch (4 us) and its partial sums a write and a read through L2 (5 TB/s).  Splits whose sums beside C do not fit the
 // context's work area are not taken: nothing is allocated here.  The most that any shape tried asks for is 69 MiB.
-// 3001 x 384, K 8192: 34 us as 3 splits against 64 us whole on the token-major kernel; 384 x 384: 16 against 64 us.
+// 3001 x 384, K 8192, one call after another: 26 us as 3 splits against 64 us whole on the token-major kernel; 384 x 384:
+// 12 against 64 us.
 void ws_dense_plan(WsArgs &a, uint32_t rows, uint32_t n, uint32_t ft, uint32_t kblocks, uint32_t clusters, bool tiled, size_t work_bytes) {
     const uint32_t nch0 = (rows + MAX_TOK - 1u) / MAX_TOK;
     uint64_t best = ~0ull;
