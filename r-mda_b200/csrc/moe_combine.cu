@@ -102,6 +102,7 @@ moe_combine_kernel(moe_combine_args a) {
         __syncthreads();
         const uint32_t terms = (PEER && a.per_gpu) ? s_terms : a.topk;
         float sg = s_f[7];
+        constexpr uint32_t TERMS = sizeof(YT) == 4 ? CB_TERMS / 2 : CB_TERMS;
         constexpr int ITS = NORM ? NORM : 1;  // unrolled where their values are kept
         float keep[ITS][V];
         float ss = 0.0f;
@@ -113,15 +114,15 @@ moe_combine_kernel(moe_combine_args a) {
                 float acc[V], f[V];
 #pragma unroll
                 for (int i = 0; i < V; i += 1) acc[i] = 0.0f;
-                for (uint32_t j0 = 0; j0 < terms; j0 += CB_TERMS) {
-                    typename moe_vec<YT, V>::raw v[CB_TERMS];
+                for (uint32_t j0 = 0; j0 < terms; j0 += TERMS) {
+                    typename moe_vec<YT, V>::raw v[TERMS];
 #pragma unroll
-                    for (uint32_t j = 0; j < CB_TERMS; j += 1) {
+                    for (uint32_t j = 0; j < TERMS; j += 1) {
                         if (j0 + j < terms && s_slot[j0 + j] != ~0u)
                             v[j] = moe_fetch<YT, V>((PEER ? s_y[j0 + j] : y) + (size_t)s_slot[j0 + j] * a.d + c);
                     }
 #pragma unroll
-                    for (uint32_t j = 0; j < CB_TERMS; j += 1) {
+                    for (uint32_t j = 0; j < TERMS; j += 1) {
                         if (j0 + j >= terms || s_slot[j0 + j] == ~0u) continue;
                         moe_floats(v[j], f);
                         moe_axpy<V>(acc, s_wt[j0 + j], f);
@@ -398,14 +399,20 @@ __device__ __forceinline__ uint2 moe_pack4(float4 v, float s) {
     return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
 }
 
-// General form: any alignment.
-__global__ void moe_cast_f16_kernel(const float *src, __half *dst, size_t n, const uint32_t *amax,
-                                    uint32_t slot) {
+// General form: any alignment, four single values in flight per thread.
+__global__ void __launch_bounds__(EL_THREADS)
+moe_cast_f16_kernel(const float *src, __half *dst, size_t n, const uint32_t *amax, uint32_t slot) {
     moe_pdl_begin();
-    float s = moe_slot_scale(amax, slot);
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        dst[i] = __float2half_rn(src[i] * s);  // cast_f16.comp:33
+    const size_t i0 = (size_t)blockIdx.x * (EL_THREADS * EL_VECS) + threadIdx.x;
+    float v[EL_VECS];
+#pragma unroll
+    for (uint32_t j = 0; j < EL_VECS; j += 1) {
+        if (i0 + j * EL_THREADS < n) v[j] = src[i0 + j * EL_THREADS];
+    }
+    const float s = moe_slot_scale(amax, slot);
+#pragma unroll
+    for (uint32_t j = 0; j < EL_VECS; j += 1) {
+        if (i0 + j * EL_THREADS < n) dst[i0 + j * EL_THREADS] = __float2half_rn(v[j] * s);  // cast_f16.comp:33
     }
 }
 
@@ -440,9 +447,8 @@ extern "C" void moe_cuda_cast_f16(moe_cuda_ctx_t *c, const float *src, void *dst
         MOE_LAUNCHED(c);
         return;
     }
-    uint32_t blocks = (uint32_t)(((uint64_t)pc.n + 255u) / 256u);
-    if (blocks > (uint32_t)c->sm_count * 16u) blocks = (uint32_t)c->sm_count * 16u;
-    moe_run(c, moe_cast_f16_kernel, blocks, 256, 0, src, (__half *)dst, pc.n, amax, pc.slot);
+    const uint32_t per = EL_VECS * EL_THREADS, blocks = (uint32_t)(((uint64_t)pc.n + per - 1u) / per);
+    moe_run(c, moe_cast_f16_kernel, blocks, EL_THREADS, 0, src, (__half *)dst, pc.n, amax, pc.slot);
     MOE_LAUNCHED(c);
 }
 

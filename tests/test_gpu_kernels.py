@@ -196,7 +196,8 @@ def _check_mm(ctx, oracle, mc, m, n, k, E, sa):
 
 
 @pytest.mark.parametrize("rows,E,K,d,shared,hc", [(512, 8, 2, 256, False, 1), (300, 128, 8, 2048, True, 1),
-                                                   (64, 16, 4, 520, True, 4), (1, 4, 4, 8, False, 1)])
+                                                   (64, 16, 4, 520, True, 4), (1, 4, 4, 8, False, 1),
+                                                   (17, 16, 5, 264, False, 1), (9, 32, 10, 2048, True, 3)])
 def test_combine(ctx, oracle, rows, E, K, d, shared, hc):
     rng = np.random.default_rng(rows + d)
     M = oracle.moe_rows(rows, K, E)
