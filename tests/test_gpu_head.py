@@ -16,7 +16,8 @@ def _f16(rng, shape, std):
 
 @pytest.mark.parametrize("rows,groups,gsize,op", [(37, 4, 256, 0), (5, 1, 2048, 0), (64, 4, 200, 1), (1, 3, 7, 0),
                                                    (3, 2, 2052, 0), (2, 1, 4096, 1), (2, 1, 4100, 0), (5, 3, 4, 0),
-                                                   (3, 1, 8192, 0), (2, 1, 8196, 1), (3, 1, 8190, 0)])
+                                                   (3, 1, 8192, 0), (2, 1, 8196, 1), (3, 1, 8190, 0),
+                                                   (1200, 1, 2050, 0), (600, 2, 1023, 0), (1300, 1, 7, 1)])
 def test_norm(ctx, oracle, rows, groups, gsize, op):
     rng = np.random.default_rng(rows + gsize)
     x = rng.standard_normal((rows, groups * gsize)).astype(np.float32) * 3.0
