@@ -42,6 +42,6 @@ def test_early_kernel_waits_and_loads_plainly(name):
     source, params, body = KERNELS[name]
     assert "moe_pdl_begin();" in body
     assert "__restrict__" not in params
-    helpers = [] if source in ("moe_ep.cu", "moe_kd.cu") else [SOURCES[source]]   # those two also hold kernels of serial launches
+    helpers = [] if source == "moe_ep.cu" else [SOURCES[source]]   # that one also holds kernels of serial launches
     for text in [body, SOURCES["moe_common.cuh"], SOURCES["moe_tc.cuh"]] + helpers:
         assert "__ldg(" not in text and "global.nc" not in text
